@@ -193,6 +193,7 @@ struct TileSet {
 // A row-ordered triangular operator and its dependency levels.  A sweep
 // (one launch) hands out chunks of at most 32 rows of one level, in level
 // order, from a ticket counter.
+struct TilePair;
 struct LevelSchedule {
     int n = 0;
     int num_levels = 0;
@@ -265,6 +266,7 @@ struct mtjg_precond {
     double *diagv = nullptr;            // R_ii
     mtjg::LevelSchedule lo;             // ILU: L solve; ICC: R' solve
     mtjg::LevelSchedule up;             // U / R solve (rows descending)
+    struct mtjg::TilePair *tile = nullptr;  // both sweeps by tiles of lines (lines.cu), in place of lo and up
     double *y = nullptr;                // temporary of apply
     double *d_b = nullptr, *d_x = nullptr;  // host-call staging
     void *trans = nullptr;              // ILU / ILUT transApply operators, built on first use

@@ -1,0 +1,963 @@
+// lines.cu -- triangular sweeps by tiles of lines.
+//
+// A level-scheduled sweep hands every level's values through the L2: about
+// 950 cycles from one SM's store to another's poll, on every level, so a
+// 96^3 grid's 286 levels took 273 (L) and 361 us (U).  The rows of a grid in its
+// natural order form lines (runs of consecutive rows, each reading the one
+// before), and the lines form planes.  Here a CTA owns a tile of lines, one
+// lane per line, and walks the levels: a value read inside the tile comes
+// from shared memory one block barrier later, and only the tile's edges go
+// through the L2, once per tile boundary on the longest path instead of once
+// per level.  What bounds a sweep then is the arithmetic of one row per
+// level: a warp's FP64 instruction holds its quarter of the SM for 64 cycles
+// on GB300, whatever its active lanes, so an L step of three entries takes
+// 4 x 64 cycles and the barrier, and a tile has 128 lanes (a warp on each
+// quarter; the diagonal's reciprocal, made once with the factor, spares the
+// U step the 563 cycles of an FP64 division).
+//
+// The sweeps' vectors are in plan order (the rows of one step next to each
+// other), so that b arrives by bulk copies, a step's x leaves in whole
+// sectors and the CTAs' polls touch few lines; one launch permutes b ahead of
+// the first sweep and one takes x back after the second.
+//
+// Each row's operations and their order are those of the ticket sweep
+// (precond.cu).  A CTA takes its rows in level order, waits on rows of lower
+// levels only, and all CTAs run at once (a cooperative launch), so the sweep
+// cannot deadlock: the lowest unfinished level is always free to run.
+#include <algorithm>
+#include <vector>
+
+#include "lines.cuh"
+#include "spmv.cuh"
+#include "sweep.cuh"
+
+namespace mtjg {
+
+constexpr int kRing = 8;          // steps whose x a tile keeps in shared memory
+constexpr int kLineK = 4;         // entries per row a record may hold
+constexpr int kMinLine = 4;       // rows per line, on average, that make lines worth it
+constexpr long long kLineSpin = 1LL << 22;
+
+// Slots of the operand pipeline (steps ahead of the arithmetic) and loader
+// warps; an FP32 step is some 150 cycles, an FP64 step 350 to 550, against
+// about 1000 for a record from memory or a value from another SM.
+template <class V>
+struct LinePipe {
+    static constexpr int kSlots = sizeof(V) == 8 ? 8 : 16;
+    static constexpr int kLoaders = sizeof(V) == 8 ? 4 : 8;
+};
+
+template <class V>
+__host__ __device__ constexpr int line_record(int kmax, int lanes)
+{
+    return lanes * ((kmax + 2) * (int)sizeof(V) + 16);
+}
+// Shared memory: the values a lane may read after a step's barrier -- the
+// ring (kRing steps of x), a zero, the entries from other CTAs (kSlots steps)
+// -- then kSlots slots of a record and b each.  An entry's code is the byte
+// offset of its value in there.
+template <class V>
+__host__ __device__ constexpr int line_zero(int lanes) { return kRing * lanes * (int)sizeof(V); }
+template <class V>
+__host__ __device__ constexpr int line_remote(int kmax, int lanes, int s)  // step s of the sweep
+{
+    return line_zero<V>(lanes) + 16 + (s % LinePipe<V>::kSlots) * kmax * lanes * (int)sizeof(V);
+}
+template <class V>
+__host__ __device__ constexpr int line_slots(int kmax, int lanes)
+{
+    return line_zero<V>(lanes) + 16 + LinePipe<V>::kSlots * kmax * lanes * (int)sizeof(V);
+}
+template <class V>
+__host__ __device__ constexpr int line_slot(int kmax, int lanes)
+{
+    return line_record<V>(kmax, lanes) + lanes * (int)sizeof(V);
+}
+template <class V>
+constexpr int line_smem(int kmax, int lanes)
+{
+    return line_slots<V>(kmax, lanes) + LinePipe<V>::kSlots * line_slot<V>(kmax, lanes);
+}
+
+// ------------------------------------------------------------ the plan
+__device__ __forceinline__ void tri_range(const TriOp &op, int i, int &b, int &e)
+{
+    b = op.range == 2 ? op.diag[i] + 1 : op.rp[i];
+    e = op.range == 1 ? op.diag[i] : op.rp[i + 1];
+}
+
+// start[i] = 1 when row i begins a line: its last entry is not row i - 1
+__global__ void k_line_start(TriOp op, int *start)
+{
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < op.n; i += gridDim.x * blockDim.x) {
+        int b, e;
+        tri_range(op, i, b, e);
+        start[i] = !(e > b && op.ci[e - 1] == i - 1);
+    }
+}
+
+// line_of from the scan of start; each line's first row
+__global__ void k_line_of(int n, const int *start, const int *scan, int *line_of, int *first, int lines)
+{
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const int l = scan[i] + start[i] - 1;
+        line_of[i] = l;
+        if (start[i]) first[l] = i;
+        if (i == 0) first[lines] = n;
+    }
+}
+
+// pstart[l] = 0 when line l continues line l - 1's plane: one of its rows
+// reads that line (pstart is 1 before)
+__global__ void k_plane_start(TriOp op, const int *line_of, int *pstart)
+{
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < op.n; i += gridDim.x * blockDim.x) {
+        int b, e;
+        tri_range(op, i, b, e);
+        const int l = line_of[i];
+        for (int k = b; k < e; ++k)
+            if (line_of[op.ci[k]] == l - 1) pstart[l] = 0;
+    }
+}
+
+__global__ void k_fill(int n, int *p, int v)
+{
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) p[i] = v;
+}
+
+// each plane's first line, and the most lines of a plane
+__global__ void k_plane_first(int lines, const int *pstart, const int *scan, int *pfirst, int planes)
+{
+    for (int l = blockIdx.x * blockDim.x + threadIdx.x; l < lines; l += gridDim.x * blockDim.x) {
+        if (pstart[l]) pfirst[scan[l]] = l;
+        if (l == 0) pfirst[planes] = lines;
+    }
+}
+
+__global__ void k_plane_long(int planes, const int *pfirst, int *longest)
+{
+    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < planes; p += gridDim.x * blockDim.x)
+        atomicMax(longest, pfirst[p + 1] - pfirst[p]);
+}
+
+// tiles of tq lines of a plane by tp planes
+__global__ void k_line_tile(int lines, const int *pstart, const int *scan, const int *pfirst, int tq, int tp, int ntq,
+                            int *part_of, int *lane_of)
+{
+    for (int l = blockIdx.x * blockDim.x + threadIdx.x; l < lines; l += gridDim.x * blockDim.x) {
+        const int p = scan[l] + pstart[l] - 1, q = l - pfirst[p];
+        part_of[l] = (p / tp) * ntq + q / tq;
+        lane_of[l] = (p % tp) * tq + q % tq;
+    }
+}
+
+__device__ __forceinline__ int ld_relaxed_int(const int *p)
+{
+    int v;
+    asm volatile("ld.relaxed.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+
+// Dependency levels, a lane per line (level is -1 before).  A line reads
+// earlier lines only and warps take lines in order from a ticket counter, so
+// every line a lane waits on is its own warp's or a running or finished
+// warp's; the lanes of a warp poll together and each round moves every lane
+// whose row is ready, so lanes may wait on each other.
+__global__ void k_line_levels(TriOp op, int lines, const int *first, int *level, unsigned *ticket, int *err)
+{
+    const int lane = threadIdx.x & 31;
+    for (;;) {
+        unsigned base = 0;
+        if (lane == 0) base = atomicAdd(ticket, 32u);
+        base = __shfl_sync(0xffffffffu, base, 0);
+        if (base >= (unsigned)lines) return;
+        const int l = (int)base + lane;
+        int i = l < lines ? first[l] : 0;
+        const int end = l < lines ? first[l + 1] : 0;
+        int own = -1;  // the level of the line's previous row
+        int c[kLineK], nx[kLineK];
+        auto load = [&](int r, int *cc) {
+            int b = 0, e = 0;
+            if (r < end) tri_range(op, r, b, e);
+#pragma unroll
+            for (int k = 0; k < kLineK; ++k) cc[k] = b + k < e ? op.ci[b + k] : -1;
+        };
+        load(i, c);
+        load(i + 1, nx);
+        long long idle = 0;
+        while (__any_sync(0xffffffffu, i < end)) {
+            bool moved = false;
+            if (i < end) {
+                int lv = 0;
+                bool ready = true;
+#pragma unroll
+                for (int k = 0; k < kLineK; ++k) {
+                    if (c[k] < 0) continue;
+                    const int d = c[k] == i - 1 ? own : ld_relaxed_int(level + c[k]);
+                    if (d < 0) ready = false;
+                    lv = max(lv, d + 1);
+                }
+                if (ready) {
+                    asm volatile("st.relaxed.gpu.global.b32 [%0], %1;" ::"l"(level + i), "r"(lv) : "memory");
+                    own = lv;
+                    i += 1;
+                    moved = true;
+#pragma unroll
+                    for (int k = 0; k < kLineK; ++k) c[k] = nx[k];
+                    load(i + 1, nx);
+                }
+            }
+            idle = __any_sync(0xffffffffu, moved) ? 0 : idle + 1;
+            if (idle > kLineSpin || ((idle & 1023) == 1023 && *(volatile int *)err)) {
+                if (lane == 0) atomicExch(err, 1);
+                return;
+            }
+        }
+    }
+}
+
+// each part's lowest and highest level (a line's levels grow along it)
+__global__ void k_part_span(int lines, const int *first, const int *part_of, const int *level, int *lo, int *hi)
+{
+    for (int l = blockIdx.x * blockDim.x + threadIdx.x; l < lines; l += gridDim.x * blockDim.x) {
+        atomicMin(lo + part_of[l], level[first[l]]);
+        atomicMax(hi + part_of[l], level[first[l + 1] - 1]);
+    }
+}
+
+// each row's position, and the row at each position (row is -1 before)
+__global__ void k_line_place(int n, int lanes, const int *line_of, const int *part_of, const int *lane_of,
+                             const int *level, const int *part_min, const int *part_step, int *pos, int *row)
+{
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const int l = line_of[i], p = part_of[l];
+        const int at = (part_step[p] + level[i] - part_min[p]) * lanes + lane_of[l];
+        pos[i] = at;
+        row[at] = i;
+    }
+}
+
+// *bad = 1 unless every entry (i, c) of `op` has its mirror (c, i) in `other`;
+// kmax: the longest row (over kLineK rules the plan out)
+__global__ void k_mirrored(TriOp op, TriOp other, int *kmax, int *bad)
+{
+    int km = 0;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < op.n; i += gridDim.x * blockDim.x) {
+        int b, e;
+        tri_range(op, i, b, e);
+        km = max(km, e - b);
+        for (int k = b; k < e && e - b <= kLineK; ++k) {
+            int b2, e2;
+            tri_range(other, op.ci[k], b2, e2);
+            bool found = false;
+            for (int q = b2; q < e2 && e2 - b2 <= kLineK; ++q) found |= other.ci[q] == i;
+            if (!found) *bad = 1;
+        }
+    }
+    for (int off = 16; off > 0; off >>= 1) km = max(km, __shfl_down_sync(0xffffffffu, km, off));
+    if ((threadIdx.x & 31) == 0) atomicMax(kmax, km);
+}
+
+// The part that holds a step: part_step is ascending (binary search).
+__device__ __forceinline__ int part_at(const int *part_step, int parts, int step)
+{
+    int lo = 0, hi = parts - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (part_step[mid] <= step) lo = mid;
+        else hi = mid - 1;
+    }
+    return lo;
+}
+
+// The entry codes of every position (without a row every code is the zero's)
+// and, with `rem`, the remote entries of each step: rem_max places a step,
+// (-1, 0) before; cursor counts a step's entries, beyond rem_max too.
+template <class V>
+__global__ void k_line_codes(TriOp op, TilePlan tp, unsigned char *rec, int *cursor, int2 *rem, int rem_max)
+{
+    const int T = tp.lanes, K = tp.kmax, bytes = line_record<V>(K, T);
+    for (int at = blockIdx.x * blockDim.x + threadIdx.x; at < tp.steps * T; at += gridDim.x * blockDim.x) {
+        const int i = tp.row[at], step = at / T, lane = at % T;
+        int code[kLineK];
+        for (int k = 0; k < kLineK; ++k) code[k] = line_zero<V>(T);
+        if (i >= 0) {
+            const int part = part_at(tp.part_step, tp.parts, step);
+            const int first = tp.part_step[part], last = tp.part_step[part + 1];
+            // the step in the sweep's order
+            auto order = [&](int s) { return op.desc ? last - 1 - s : s - first; };
+            int b, e;
+            tri_range(op, i, b, e);
+            for (int k = 0; k < e - b; ++k) {
+                const int c = tp.pos[op.ci[op.mode == 3 ? e - 1 - k : b + k]], cs = c / T;
+                if (cs >= first && cs < last && order(step) - order(cs) < kRing) {
+                    code[k] = ((order(cs) % kRing) * T + c % T) * (int)sizeof(V);
+                } else {
+                    code[k] = line_remote<V>(K, T, order(step)) + (k * T + lane) * (int)sizeof(V);
+                    if (rem) {
+                        const int q = atomicAdd(cursor + step, 1);
+                        if (q < rem_max) rem[(size_t)step * rem_max + q] = make_int2(c, k * T + lane);
+                    }
+                }
+            }
+        }
+        reinterpret_cast<int4 *>(rec + (size_t)step * bytes + (size_t)T * (K + 2) * sizeof(V))[lane] =
+            make_int4(code[0], code[1], code[2], code[3]);
+    }
+}
+
+// The values of every position: entries in the order the sweep adds them,
+// the diagonal and its reciprocal (1 and 1 without a row).  A row with fewer
+// entries is filled up with ones whose product with the zero is -0, which
+// leaves every sum as it is.
+template <class V>
+__global__ void k_line_values(TriOp op, TilePlan tp, unsigned char *rec, const V *v, const V *diagv)
+{
+    const int T = tp.lanes, K = tp.kmax, bytes = line_record<V>(K, T);
+    for (int at = blockIdx.x * blockDim.x + threadIdx.x; at < tp.steps * T; at += gridDim.x * blockDim.x) {
+        const int i = tp.row[at], lane = at % T;
+        V *rv = reinterpret_cast<V *>(rec + (size_t)(at / T) * bytes);
+        int b = 0, e = 0;
+        V d = V(1);
+        if (i >= 0) {
+            tri_range(op, i, b, e);
+            if (op.mode == 1) d = v[op.diag[i]];
+            if (op.mode == 2) d = diagv[i];
+        }
+        const V fill = op.mode >= 2 ? V(0) : -V(0);  // modes 2 and 3 subtract
+        for (int k = 0; k < K; ++k) rv[k * T + lane] = k < e - b ? v[op.mode == 3 ? e - 1 - k : b + k] : fill;
+        rv[K * T + lane] = d;
+        // the reciprocal, or 0 where a quotient by d needs a real division
+        const V m = fabs(d);
+        const bool safe = sizeof(V) == 8 ? m > V(1e-90) && m < V(1e90) : m > V(1e-12) && m < V(1e12);
+        rv[(K + 1) * T + lane] = safe ? V(1) / d : V(0);
+    }
+}
+
+// ------------------------------------------------------------ the sweeps
+// b into plan order, and the two sweeps' outputs to pending.
+template <class V>
+__global__ void k_tile_in(int count, const int *row, const V *b, V *bp, V *yp, V *xp, const int *status)
+{
+    if (status && *status != ST_RUNNING) return;
+    const V p = pending_value<V>();
+    for (int at = blockIdx.x * blockDim.x + threadIdx.x; at < count; at += gridDim.x * blockDim.x) {
+        const int i = row[at];
+        bp[at] = i >= 0 ? b[i] : V(0);
+        yp[at] = p;
+        xp[at] = p;
+    }
+}
+
+template <class V>
+__global__ void k_tile_out(int n, const int *pos, const V *xp, V *x, const int *status)
+{
+    if (status && *status != ST_RUNNING) return;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) x[i] = xp[pos[i]];
+}
+
+// a / d from y = RN(1 / d) by one residual correction (two in STRICT and
+// FP32): P. Markstein, "Computation of elementary functions on the IBM RISC
+// System/6000 processor", IBM J. Res. Dev. 34 (1990): with y the rounded
+// reciprocal, a faithful quotient corrected by its exact residual is the
+// rounded quotient.  The first correction makes q faithful (and the rounded
+// quotient but for about one operand pair in 2^52), the second settles it.
+// Out of the range where every intermediate is normal: a real division.
+// a real division, kept out of line: inlined, its steps were computed ahead
+// of the test on every row
+__device__ __noinline__ double full_div(double a, double d) { return a / d; }
+__device__ __noinline__ float full_div(float a, float d) { return a / d; }
+
+template <bool S>
+__device__ __forceinline__ double line_div(double a, double d, double y)
+{
+    const double q0 = a * y;
+    double q = fma(fma(-d, q0, a), y, q0);
+    if constexpr (S) q = fma(fma(-d, q, a), y, q);
+    // tested on the bits (an FP64 compare takes as long as an FMA), after the
+    // quotient: the test hides in its latency
+    const unsigned hi = (unsigned)__double2hiint(a), ea = (hi >> 20) & 0x7ffu;
+    if (ea - 623u > 800u || __double2hiint(y) == 0) {
+        const bool zero = ((hi & 0x7fffffffu) | (unsigned)__double2loint(a)) == 0u;
+        q = zero && __double2hiint(y) != 0 ? q0 : full_div(a, d);
+    }
+    return q;
+}
+
+template <bool S>
+__device__ __forceinline__ float line_div(float a, float d, float y)
+{
+    const float q0 = a * y;
+    float q = fmaf(fmaf(-d, q0, a), y, q0);
+    q = fmaf(fmaf(-d, q, a), y, q);
+    const unsigned ea = (__float_as_uint(a) >> 23) & 0xffu;
+    if (ea - 87u > 80u || y == 0.0f) q = a == 0.0f && y != 0.0f ? q0 : full_div(a, d);
+    return q;
+}
+
+__device__ __forceinline__ void mbar_arrive(uint64_t *bar)
+{
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+
+// Non-blocking (try_wait may suspend the thread).
+__device__ __forceinline__ bool mbar_test_wait(uint64_t *bar, unsigned parity)
+{
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+
+// The lanes of a part (threads 0 .. T-1) only compute: everything a step
+// needs is in shared memory by then.  One thread of the last warp keeps the
+// slots filled (bulk copies of the record and of b), and loader warp w takes
+// steps w, w + kLoaders, ...: it brings in the entries solved by other CTAs,
+// polling those still pending, so neither memory latency nor a poll's round
+// trip sits in the chain of steps.  A slot's barrier completes when its
+// copies have landed and its loader has arrived.  s_done: steps whose slots
+// the lanes have read.
+//
+// With one warp on each quarter of the SM, every instruction of the lanes'
+// loop is on the path: operands are read ahead of the step's barrier, and an
+// entry costs one shared-memory read at a prepared offset and its
+// multiply-add, with no test for where it comes from.  96^3 convection-
+// diffusion, L / U sweep in us: tickets (precond.cu) 273 / 361; register
+// prefetch by the computing warps 494 / 519 (a warp's few scoreboards make an
+// old load wait for the newer ones); loader warps, b and x in row order 211 /
+// 250 (32 sectors a warp for each); plan order, a test per entry 155 / 198;
+// prepared offsets 104 / 155; operands read inside the chain 96 / 135 (552
+// cycles an L step, of which the four dependent FP64 operations take 300).
+// A whole apply, both permutations included: 633 -> 253 us; 128^3 Poisson
+// ILU 389 -> 355 with the last step; 63^3 FP32 sweeps 248 / 239 -> 39 / 55.
+template <bool S, int MODE, int K, int T, class V>
+__global__ void __launch_bounds__(T + 32 * LinePipe<V>::kLoaders + 32, 1)
+    k_line_sweep(const unsigned char *__restrict__ rec, const int *__restrict__ part_step,
+                 const int2 *__restrict__ rem, int rem_max, const V *b, V *x, const int *status, int *err, int spin)
+{
+    constexpr int D = LinePipe<V>::kSlots, LW = LinePipe<V>::kLoaders;
+    constexpr bool kDesc = MODE == 1 || MODE == 3, kDiv = MODE == 1 || MODE == 2;
+    constexpr int kRec = line_record<V>(K, T), kSlot = line_slot<V>(K, T), kBytesB = T * (int)sizeof(V);
+    extern __shared__ __align__(128) unsigned char sm[];
+    __shared__ __align__(8) uint64_t full[D];
+    __shared__ volatile int s_done, s_abort;
+    if (status && *status != ST_RUNNING) return;
+    const int tid = (int)threadIdx.x, lane = tid & 31;
+    const int step0 = part_step[blockIdx.x], steps = part_step[blockIdx.x + 1] - step0;
+    unsigned char *slots = sm + line_slots<V>(K, T);
+    if (tid == 0) {
+        for (int i = 0; i < D; ++i) mbar_init(&full[i], 2);
+        mbar_fence_init();
+        s_done = 0;
+        s_abort = 0;
+        *reinterpret_cast<V *>(sm + line_zero<V>(T)) = V(0);
+    }
+    __syncthreads();
+    // step s of the sweep is step plan_step(s) of the plan
+    auto plan_step = [&](int s) { return step0 + (kDesc ? steps - 1 - s : s); };
+    auto give_up = [&]() {
+        s_abort = 1;
+        atomicExch(err, 1);
+    };
+    auto slot_free = [&](int s) {  // the lanes are done with step s - D
+        for (long long i = 0; s_done < s - D + 1; ++i) {
+            if (s_abort) return false;
+            if (i > kLineSpin * 4) {
+                give_up();
+                return false;
+            }
+            __nanosleep(20);
+        }
+        __threadfence_block();
+        return true;
+    };
+
+    if (tid >= T + 32 * LW) {  // the records and b
+        if (lane == 0) {
+            int s = 0;
+            for (; s < steps && slot_free(s); ++s) {
+                const size_t ps = (size_t)plan_step(s);
+                uint64_t *bar = &full[s % D];
+                unsigned char *to = slots + (s % D) * kSlot;
+                fence_proxy_async();
+                mbar_arrive_expect_tx(bar, (unsigned)(kRec + kBytesB));
+                bulk_g2s(to, rec + ps * kRec, (unsigned)kRec, bar);
+                bulk_g2s(to + kRec, b + ps * T, (unsigned)kBytesB, bar);
+            }
+            // every copy lands before the block leaves (after an abort the
+            // loaders' arrivals may be missing: a bounded wait is enough, the
+            // copies themselves take microseconds)
+            for (int t = max(0, s - D); t < s; ++t)
+                if (!mbar_wait_bounded(&full[t % D], (unsigned)(t / D) & 1u, s_abort ? 1LL << 16 : kWaitLimit)) give_up();
+        }
+    } else if (tid >= T) {  // the entries from other CTAs
+        int s = (tid - T) >> 5;
+        // step t's first items (position, slot), read ahead of its turn
+        auto look = [&](int t) {
+            return t < steps && lane < rem_max ? rem[(size_t)plan_step(t) * rem_max + lane] : make_int2(-1, 0);
+        };
+        int2 next = look(s);
+        for (; s < steps; s += LW) {
+            int2 it = next;
+            next = look(s + LW);
+            // the lanes read step s - D's entries after its barrier: one step more
+            if (!__all_sync(0xffffffffu, slot_free(s + 1))) break;
+            V *xs = reinterpret_cast<V *>(sm + line_remote<V>(K, T, s));
+            bool bad = false;
+            for (int q = lane; it.x >= 0;) {
+                xs[it.y] = wait_x(x, it.x, err, spin, bad);
+                q += 32;
+                it = q < rem_max ? rem[(size_t)plan_step(s) * rem_max + q] : make_int2(-1, 0);
+            }
+            if (bad) give_up();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&full[s % D]);
+        }
+    } else {
+        bool bad = false;
+        int slot = 0;         // of the coming step
+        unsigned parity = 0;  // of its barrier
+        struct Operands {
+            V vv[K], bi, d, y;
+            int4 code;
+        } even, odd;
+        auto fetch = [&](Operands &o, int sl) {
+            const unsigned char *at = slots + sl * kSlot;
+            const V *cv = reinterpret_cast<const V *>(at) + tid;
+            o.code = reinterpret_cast<const int4 *>(at + (K + 2) * kBytesB)[tid];
+            o.bi = reinterpret_cast<const V *>(at + kRec)[tid];
+#pragma unroll
+            for (int k = 0; k < K; ++k) o.vv[k] = cv[k * T];
+            if constexpr (kDiv) {
+                o.d = cv[K * T];
+                o.y = cv[(K + 1) * T];
+            }
+        };
+        auto wait_fetch = [&](Operands &o, int sl, unsigned par) {
+            bool ok = false;
+            for (long long i = 0; i < kWaitLimit && !ok && !bad; ++i) {
+                ok = mbar_try_wait(&full[sl], par);
+                if ((i & 255) == 255 && s_abort) break;
+            }
+            if (!ok && !bad) {
+                bad = true;
+                give_up();
+            }
+            fetch(o, sl);
+            if (bad) o.code = make_int4(line_zero<V>(T), line_zero<V>(T), line_zero<V>(T), line_zero<V>(T));
+        };
+        int prev = 0;  // the slot before it
+        V *out = x + (size_t)plan_step(0) * T + tid;
+        int here = tid * (int)sizeof(V);  // this step's place in the ring
+        // Step s on `o`.  The next step's operands are read into `next` while
+        // the sum's multiply-adds wait for each other (a straight line, for
+        // the compiler to interleave), and again after this step's x is out
+        // if their slot was not full: never waiting before that, since
+        // another CTA may need this x to fill the slot.
+        auto step = [&](int s, Operands &o, Operands &next) {
+            asm volatile("bar.sync 1, %0;" ::"n"(T) : "memory");  // step s - 1 is in the ring, step s's slot is read
+            const int at[4] = {o.code.x, o.code.y, o.code.z, o.code.w};
+            V xv[K];
+#pragma unroll
+            for (int k = 0; k < K; ++k) xv[k] = *reinterpret_cast<const V *>(sm + at[k]);
+            const int sl = slot;
+            const unsigned par = parity;
+            const bool early = mbar_test_wait(&full[sl], par);
+            // (the address waits for the test's answer: reads must not pass it)
+            fetch(next, early ? sl : prev);
+            prev = sl;
+            if (tid == 0) s_done = s + 1;
+            slot = sl + 1 == D ? 0 : sl + 1;
+            parity ^= slot == 0 ? 1u : 0u;
+            V acc = MODE >= 2 ? o.bi : V(0);
+#pragma unroll
+            for (int k = 0; k < K; ++k) acc = fmac<S>(MODE >= 2 ? -o.vv[k] : o.vv[k], xv[k], acc);
+            if constexpr (MODE <= 1) acc = o.bi - acc;
+            if constexpr (kDiv) acc = line_div<S>(acc, o.d, o.y);
+            // (the result of an operation is never the pending pattern, a signalling NaN)
+            *reinterpret_cast<V *>(sm + here) = acc;
+            st_relaxed(out, acc);
+            out += kDesc ? -T : T;
+            here = here + kBytesB >= kRing * kBytesB ? here + kBytesB - kRing * kBytesB : here + kBytesB;
+            if (!early && s + 1 < steps) wait_fetch(next, sl, par);
+        };
+        if (steps > 0) {
+            wait_fetch(even, 0, 0);
+            slot = 1;
+        }
+#pragma unroll 1
+        for (int s = 0; s < steps; s += 2) {
+            step(s, even, odd);
+            if (s + 1 < steps) step(s + 1, odd, even);
+        }
+    }
+}
+
+namespace {
+
+template <bool S, int MODE, int K, int T, class V>
+cudaError_t launch_line(mtjg_ctx *ctx, const TilePlan *tp, const TileOp &op, const V *b, V *x, const int *status,
+                        int spin)
+{
+    auto k = k_line_sweep<S, MODE, K, T, V>;
+    const int smem = line_smem<V>(K, T);
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)tp->parts);
+    cfg.blockDim = dim3(T + 32 * LinePipe<V>::kLoaders + 32);
+    cfg.dynamicSmemBytes = (size_t)smem;
+    cfg.stream = ctx->stream;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeCooperative;
+    attr.val.cooperative = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    const unsigned char *rec = sizeof(V) == 8 ? op.rec64 : op.rec32;
+    e = cudaLaunchKernelEx(&cfg, k, rec, (const int *)tp->part_step, (const int2 *)op.rem, op.rem_max, b, x, status,
+                           ctx->d_flag, spin);
+    if (e == cudaSuccess) ctx->launches++;
+    return e;
+}
+
+template <bool S, int MODE, class V>
+cudaError_t launch_k(mtjg_ctx *ctx, const TilePlan *tp, const TileOp &op, const V *b, V *x, const int *status, int spin)
+{
+    const bool wide = tp->lanes == 256;
+    switch (tp->kmax) {
+    case 2:
+        return wide ? launch_line<S, MODE, 2, 256, V>(ctx, tp, op, b, x, status, spin)
+                    : launch_line<S, MODE, 2, 128, V>(ctx, tp, op, b, x, status, spin);
+    case 3:
+        return wide ? launch_line<S, MODE, 3, 256, V>(ctx, tp, op, b, x, status, spin)
+                    : launch_line<S, MODE, 3, 128, V>(ctx, tp, op, b, x, status, spin);
+    default:
+        return wide ? launch_line<S, MODE, 4, 256, V>(ctx, tp, op, b, x, status, spin)
+                    : launch_line<S, MODE, 4, 128, V>(ctx, tp, op, b, x, status, spin);
+    }
+}
+
+template <bool S>
+cudaError_t launch_mode(mtjg_ctx *ctx, const TilePlan *tp, const TileOp &op, const double *b, double *x,
+                        const int *status, int spin)
+{
+    switch (op.mode) {
+    case 0: return launch_k<S, 0, double>(ctx, tp, op, b, x, status, spin);
+    case 1: return launch_k<S, 1, double>(ctx, tp, op, b, x, status, spin);
+    case 2: return launch_k<S, 2, double>(ctx, tp, op, b, x, status, spin);
+    default: return launch_k<S, 3, double>(ctx, tp, op, b, x, status, spin);
+    }
+}
+
+cudaError_t sweep_op(mtjg_ctx *ctx, const TilePlan *tp, const TileOp &op, bool strict, const double *b, double *x,
+                     const int *status, int spin)
+{
+    return strict ? launch_mode<true>(ctx, tp, op, b, x, status, spin)
+                  : launch_mode<false>(ctx, tp, op, b, x, status, spin);
+}
+
+// the FP32 sweeps of the mixed-precision inner solves: MODE 0 and 1, FAST
+cudaError_t sweep_op(mtjg_ctx *ctx, const TilePlan *tp, const TileOp &op, bool, const float *b, float *x,
+                     const int *status, int spin)
+{
+    return op.mode == 0 ? launch_k<false, 0, float>(ctx, tp, op, b, x, status, spin)
+                        : launch_k<false, 1, float>(ctx, tp, op, b, x, status, spin);
+}
+
+int grid_rows(mtjg_ctx *ctx, int64_t n)
+{
+    return (int)std::max<int64_t>(1, std::min<int64_t>((n + kBlock - 1) / kBlock, ctx->num_sms * 8));
+}
+
+template <class V>
+cudaError_t apply_t(mtjg_ctx *ctx, const TilePair *t, bool strict, const V *b, V *x, const int *status, int spin, V *bp,
+                    V *yp, V *xp)
+{
+    const TilePlan *tp = t->plan;
+    const int count = tp->steps * tp->lanes;
+    k_tile_in<V><<<grid_rows(ctx, count), kBlock, 0, ctx->stream>>>(count, tp->row, b, bp, yp, xp, status);
+    ctx->launches++;
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) e = sweep_op(ctx, tp, t->op[0], strict, (const V *)bp, yp, status, spin);
+    if (e == cudaSuccess) e = sweep_op(ctx, tp, t->op[1], strict, (const V *)yp, xp, status, spin);
+    if (e != cudaSuccess) return e;
+    k_tile_out<V><<<grid_rows(ctx, tp->n), kBlock, 0, ctx->stream>>>(tp->n, tp->pos, xp, x, status);
+    ctx->launches++;
+    return cudaGetLastError();
+}
+
+}  // namespace
+
+cudaError_t tile_apply(mtjg_ctx *ctx, const TilePair *t, bool strict, const double *b, double *x, const int *status,
+                       int spin)
+{
+    return apply_t<double>(ctx, t, strict, b, x, status, spin, t->plan->b64, t->plan->y64, t->plan->x64);
+}
+
+cudaError_t tile_apply(mtjg_ctx *ctx, const TilePair *t, bool strict, const float *b, float *x, const int *status,
+                       int spin)
+{
+    return apply_t<float>(ctx, t, strict, b, x, status, spin, t->plan->b32, t->plan->y32, t->plan->x32);
+}
+
+static void free_plan(TilePlan *&tp)
+{
+    if (!tp) return;
+    cudaFree(tp->part_step);
+    cudaFree(tp->pos);
+    cudaFree(tp->row);
+    cudaFree(tp->b64);
+    cudaFree(tp->b32);
+    delete tp;
+    tp = nullptr;
+}
+
+void free_tiles_of(TilePair *&t)
+{
+    if (!t) return;
+    if (t->owns_plan) free_plan(t->plan);
+    for (TileOp &op : t->op) {
+        cudaFree(op.rec64);
+        cudaFree(op.rec32);
+        cudaFree(op.rem);
+    }
+    delete t;
+    t = nullptr;
+}
+
+// Tiles of lines pay when rows form lines (kMinLine rows each on average), a
+// record holds every row (kLineK entries), the two triangles mirror each
+// other (so that one plan, walked up and down, serves both sweeps), the tiles
+// fit the SMs one each (none waits for a place), and the empty lanes stay
+// fewer than the rows.  Tiles: 128 lanes, 256 when 128 give more tiles than
+// SMs; among the shapes the one with the fewest tile boundaries on a path
+// across the grid.
+static int tile_plan(mtjg_ctx *ctx, const TriOp &op, const TriOp &up, TilePlan **out)
+{
+    *out = nullptr;
+    const int n = op.n;
+    int coop = 0;
+    if (n == 0 || cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, ctx->device) != cudaSuccess || !coop)
+        return MTJG_OK;
+    TilePlan *tp = new TilePlan();
+    tp->n = n;
+    int *work = nullptr, *lw = nullptr, *pw = nullptr;
+    auto done = [&](int st, bool keep) {
+        cudaFree(work);
+        cudaFree(lw);
+        cudaFree(pw);
+        if (keep) *out = tp;
+        else free_plan(tp);
+        return st;
+    };
+#define LP_CUDA(call)                                                           \
+    do {                                                                        \
+        cudaError_t e_ = (call);                                                \
+        if (e_ != cudaSuccess) return done(cuda_fail(e_, "sweep plan"), false); \
+    } while (0)
+    cudaStream_t q = ctx->stream;
+    const int g = grid_rows(ctx, n);
+    LP_CUDA(cudaMalloc(&work, sizeof(int) * (4 * (size_t)n + 2 + 4)));
+    int *start = work, *scan = start + n, *line_of = scan + n + 1, *level = line_of + n, *scalars = level + n;
+    // scalars: longest row, lines of the longest plane, ticket, 1 unless mirrored
+    LP_CUDA(cudaMemsetAsync(scalars, 0, sizeof(int) * 4, q));
+    k_line_start<<<g, kBlock, 0, q>>>(op, start);
+    k_mirrored<<<g, kBlock, 0, q>>>(op, up, scalars, scalars + 3);
+    k_mirrored<<<g, kBlock, 0, q>>>(up, op, scalars, scalars + 3);
+    ctx->launches += 3;
+    int st = exclusive_scan(ctx, start, scan, n);
+    if (st != MTJG_OK) return done(st, false);
+    int lines = 0, sc[4] = {};
+    LP_CUDA(cudaMemcpyAsync(&lines, scan + n, sizeof(int), cudaMemcpyDeviceToHost, q));
+    LP_CUDA(cudaMemcpyAsync(sc, scalars, sizeof(sc), cudaMemcpyDeviceToHost, q));
+    LP_CUDA(cudaStreamSynchronize(q));
+    tp->kmax = sc[0] == 1 ? 2 : sc[0];
+    if (tp->kmax < 2 || tp->kmax > kLineK || sc[3] || (int64_t)lines * kMinLine > n) return done(MTJG_OK, false);
+    // first row of each line, plane starts and their scan, first line of each plane, part and lane
+    LP_CUDA(cudaMalloc(&lw, sizeof(int) * (6 * (size_t)lines + 4)));
+    int *first = lw, *pstart = first + lines + 1, *pscan = pstart + lines, *pfirst = pscan + lines + 1;
+    int *part_of = pfirst + lines + 1, *lane_of = part_of + lines;
+    const int gl = grid_rows(ctx, lines);
+    k_line_of<<<g, kBlock, 0, q>>>(n, start, scan, line_of, first, lines);
+    k_fill<<<gl, kBlock, 0, q>>>(lines, pstart, 1);
+    k_plane_start<<<g, kBlock, 0, q>>>(op, line_of, pstart);
+    ctx->launches += 3;
+    st = exclusive_scan(ctx, pstart, pscan, lines);
+    if (st != MTJG_OK) return done(st, false);
+    int planes = 0, longest = 0;
+    LP_CUDA(cudaMemcpyAsync(&planes, pscan + lines, sizeof(int), cudaMemcpyDeviceToHost, q));
+    LP_CUDA(cudaStreamSynchronize(q));
+    k_plane_first<<<gl, kBlock, 0, q>>>(lines, pstart, pscan, pfirst, planes);
+    k_plane_long<<<grid_rows(ctx, planes), kBlock, 0, q>>>(planes, pfirst, scalars + 1);
+    ctx->launches += 2;
+    LP_CUDA(cudaMemcpyAsync(&longest, scalars + 1, sizeof(int), cudaMemcpyDeviceToHost, q));
+    LP_CUDA(cudaStreamSynchronize(q));
+    int tq = 0, ntq = 0, best = 0;
+    for (int T = 128; T <= 256 && !tp->parts; T *= 2)
+        for (int a = 1; a <= T; a *= 2) {
+            const int64_t nq = (longest + a - 1) / a, np = (planes + T / a - 1) / (T / a);
+            if (nq * np > ctx->num_sms || (tp->parts && nq + np >= best)) continue;
+            tp->parts = (int)(nq * np);
+            tp->lanes = T;
+            tq = a;
+            ntq = (int)nq;
+            best = (int)(nq + np);
+        }
+    int optin = 0;
+    LP_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
+    if (!tp->parts || line_smem<double>(tp->kmax, tp->lanes) + 1024 > optin ||
+        line_smem<float>(tp->kmax, tp->lanes) + 1024 > optin)
+        return done(MTJG_OK, false);
+    const int P = tp->parts, T = tp->lanes;
+    LP_CUDA(cudaMalloc(&pw, sizeof(int) * 2 * (size_t)P));
+    LP_CUDA(cudaMalloc(&tp->part_step, sizeof(int) * (size_t)(P + 1)));
+    LP_CUDA(cudaMalloc(&tp->pos, sizeof(int) * (size_t)n));
+    k_line_tile<<<gl, kBlock, 0, q>>>(lines, pstart, pscan, pfirst, tq, T / tq, ntq, part_of, lane_of);
+    LP_CUDA(cudaMemsetAsync(level, 0xff, sizeof(int) * (size_t)n, q));
+    LP_CUDA(cudaMemsetAsync(ctx->d_flag, 0, sizeof(int), q));
+    const int warps = (lines + 31) / 32;
+    k_line_levels<<<std::max(1, std::min((warps + 3) / 4, ctx->num_sms * 8)), 128, 0, q>>>(
+        op, lines, first, level, reinterpret_cast<unsigned *>(scalars + 2), ctx->d_flag);
+    k_fill<<<1, kBlock, 0, q>>>(P, pw, 0x7fffffff);
+    k_fill<<<1, kBlock, 0, q>>>(P, pw + P, -1);
+    k_part_span<<<gl, kBlock, 0, q>>>(lines, first, part_of, level, pw, pw + P);
+    ctx->launches += 5;
+    std::vector<int> span(2 * (size_t)P), step((size_t)P + 1, 0);
+    int flag = 0;
+    LP_CUDA(cudaMemcpyAsync(span.data(), pw, sizeof(int) * 2 * (size_t)P, cudaMemcpyDeviceToHost, q));
+    LP_CUDA(cudaMemcpyAsync(&flag, ctx->d_flag, sizeof(int), cudaMemcpyDeviceToHost, q));
+    LP_CUDA(cudaStreamSynchronize(q));
+    if (flag) {
+        cudaMemset(ctx->d_flag, 0, sizeof(int));
+        return done(fail(MTJG_ERR_DEVICE_TIMEOUT, "level analysis: a bounded wait gave up"), false);
+    }
+    int64_t steps = 0;
+    for (int p = 0; p < P; ++p) {
+        const int lo = span[(size_t)p], hi = span[(size_t)(P + p)];
+        steps += hi >= lo ? hi - lo + 1 : 0;
+        if (steps * T > 2 * (int64_t)n + 65536) return done(MTJG_OK, false);
+        step[(size_t)p + 1] = (int)steps;
+    }
+    tp->steps = (int)steps;
+    const size_t count = (size_t)steps * T;
+    LP_CUDA(cudaMemcpyAsync(tp->part_step, step.data(), sizeof(int) * (size_t)(P + 1), cudaMemcpyHostToDevice, q));
+    LP_CUDA(cudaMalloc(&tp->row, sizeof(int) * count));
+    LP_CUDA(cudaMemsetAsync(tp->row, 0xff, sizeof(int) * count, q));
+    k_line_place<<<g, kBlock, 0, q>>>(n, T, line_of, part_of, lane_of, level, pw, tp->part_step, tp->pos, tp->row);
+    ctx->launches++;
+    LP_CUDA(cudaMalloc(&tp->b64, sizeof(double) * 3 * count));
+    tp->y64 = tp->b64 + count;
+    tp->x64 = tp->y64 + count;
+    // a launch that has nothing to do (a status other than running) tells
+    // whether the device takes this cooperative grid
+    static_assert(ST_RUNNING != -1, "the trial launch's status");
+    LP_CUDA(cudaMemsetAsync(scalars, 0xff, sizeof(int), q));
+    TileOp none;
+    none.mode = 1;
+    const cudaError_t e = sweep_op(ctx, tp, none, false, (const double *)nullptr, (double *)nullptr, scalars, 0);
+    if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported) {
+        (void)cudaGetLastError();
+        return done(MTJG_OK, false);
+    }
+    LP_CUDA(e);
+    LP_CUDA(cudaStreamSynchronize(q));
+    return done(MTJG_OK, true);
+}
+#undef LP_CUDA
+
+// A sweep's entry codes and the lists of what it reads from other parts: 32
+// places a step (a tile of 8 x 16 lines of a grid needs at most 24), or as
+// many as the longest needs.
+__global__ void k_most(int n, const int *v, int *most)
+{
+    int m = 0;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) m = max(m, v[i]);
+    for (int off = 16; off > 0; off >>= 1) m = max(m, __shfl_down_sync(0xffffffffu, m, off));
+    if ((threadIdx.x & 31) == 0) atomicMax(most, m);
+}
+
+static int tile_op(mtjg_ctx *ctx, const TilePlan *tp, const TriOp &op, TileOp &out)
+{
+    out.mode = op.mode;
+    cudaStream_t q = ctx->stream;
+    const int S = tp->steps, g = grid_rows(ctx, (int64_t)S * tp->lanes);
+    int *cursor = nullptr;
+    MTJG_CUDA(cudaMalloc(&out.rec64, (size_t)S * line_record<double>(tp->kmax, tp->lanes)));
+    MTJG_CUDA(cudaMalloc(&cursor, sizeof(int) * (size_t)(S + 1)));
+    cudaError_t e = cudaSuccess;
+    int most = 32;
+    do {
+        out.rem_max = most;
+        cudaFree(out.rem);
+        out.rem = nullptr;
+        const size_t bytes = sizeof(int2) * (size_t)S * most;
+        if ((e = cudaMalloc(&out.rem, bytes)) != cudaSuccess) break;
+        cudaMemsetAsync(out.rem, 0xff, bytes, q);
+        cudaMemsetAsync(cursor, 0, sizeof(int) * (size_t)(S + 1), q);
+        k_line_codes<double><<<g, kBlock, 0, q>>>(op, *tp, out.rec64, cursor, (int2 *)out.rem, most);
+        k_most<<<grid_rows(ctx, S), kBlock, 0, q>>>(S, cursor, cursor + S);
+        ctx->launches += 2;
+        e = cudaMemcpyAsync(&most, cursor + S, sizeof(int), cudaMemcpyDeviceToHost, q);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(q);
+    } while (e == cudaSuccess && most > out.rem_max);
+    cudaFree(cursor);
+    if (e != cudaSuccess) return cuda_fail(e, "sweep plan");
+    return MTJG_OK;
+}
+
+int tile_pair(mtjg_ctx *ctx, const TriOp &lo, const TriOp &up, TilePlan *plan, TilePair **out)
+{
+    *out = nullptr;
+    TilePair *t = new TilePair();
+    t->owns_plan = plan == nullptr;
+    t->plan = plan;
+    int st = MTJG_OK;
+    if (!plan) st = tile_plan(ctx, lo, up, &t->plan);
+    if (st == MTJG_OK && t->plan) {
+        st = tile_op(ctx, t->plan, lo, t->op[0]);
+        if (st == MTJG_OK) st = tile_op(ctx, t->plan, up, t->op[1]);
+    }
+    if (st != MTJG_OK || !t->plan) free_tiles_of(t);
+    else *out = t;
+    return st;
+}
+
+int tile_values(mtjg_ctx *ctx, TilePair *t, int which, const TriOp &op, const double *v, const double *diagv)
+{
+    const TilePlan *tp = t->plan;
+    k_line_values<double><<<grid_rows(ctx, (int64_t)tp->steps * tp->lanes), kBlock, 0, ctx->stream>>>(
+        op, *tp, t->op[which].rec64, v, diagv);
+    ctx->launches++;
+    MTJG_CUDA(cudaGetLastError());
+    return MTJG_OK;
+}
+
+int tile_values(mtjg_ctx *ctx, TilePair *t, int which, const TriOp &op, const float *v, const float *diagv)
+{
+    TilePlan *tp = t->plan;
+    TileOp &to = t->op[which];
+    const size_t count = (size_t)tp->steps * tp->lanes;
+    if (!tp->b32) {
+        MTJG_CUDA(cudaMalloc(&tp->b32, sizeof(float) * 3 * count));
+        tp->y32 = tp->b32 + count;
+        tp->x32 = tp->y32 + count;
+    }
+    if (!to.rec32) {
+        const size_t bytes = (size_t)tp->steps * line_record<float>(tp->kmax, tp->lanes);
+        MTJG_CUDA(cudaMalloc(&to.rec32, bytes));
+        k_line_codes<float><<<grid_rows(ctx, (int64_t)count), kBlock, 0, ctx->stream>>>(
+            op, *tp, to.rec32, nullptr, nullptr, 0);
+        ctx->launches++;
+    }
+    k_line_values<float><<<grid_rows(ctx, (int64_t)count), kBlock, 0, ctx->stream>>>(op, *tp, to.rec32, v, diagv);
+    ctx->launches++;
+    MTJG_CUDA(cudaGetLastError());
+    return MTJG_OK;
+}
+
+}  // namespace mtjg

@@ -8,6 +8,9 @@
 // counting sort, stable in row index) and cut into chunks of at most 32 rows
 // of one level.
 //
+// ILU, ICC and ILU's transposed solves take tiles of lines (lines.cu) where
+// the factor's rows form lines; what follows is every other triangular solve.
+//
 // A triangular solve is one launch (k_trsv_sweep).  Its output vector is
 // first filled with kPending, a signalling NaN that no arithmetic produces
 // (an operation on a signalling NaN returns a quiet one).  Warps take chunks
@@ -24,7 +27,9 @@
 #include <cstdlib>
 #include <cstring>
 
+#include "lines.cuh"
 #include "spmv.cuh"
+#include "sweep.cuh"
 
 namespace mtjg {
 
@@ -179,13 +184,6 @@ __global__ void k_ilu_level(const int *perm, int beg, int cnt, const int *rp, co
 }
 
 // ---------------------------------------------------- triangular sweeps
-// x entries not yet solved hold this signalling NaN (FP64; kPending32 in the
-// FP32 sweeps of the mixed-precision inner solves).
-constexpr unsigned long long kPending = 0x7FF40000DEADBEEFull;
-constexpr unsigned long long kQuietNaN = 0x7FF8000000000000ull;
-constexpr unsigned kPending32 = 0x7FA0BEEFu;
-constexpr unsigned kQuietNaN32 = 0x7FC00000u;
-constexpr long long kSweepSpinLimit = 1LL << 21;
 constexpr int kSweepBlock = 128;
 // warps per SM a sweep launches, and polls of a pending entry before the
 // poller starts to sleep between polls; both can be set in the environment
@@ -212,43 +210,6 @@ static bool sweep_lookahead(int mode, int dflt)
     return (env_int("MTJG_SWEEP_LOOKAHEAD", dflt, 0, 7) >> mode) & 1;
 }
 
-__device__ __forceinline__ double ld_relaxed(const double *p)
-{
-    unsigned long long v;
-    asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-    return __longlong_as_double((long long)v);
-}
-
-__device__ __forceinline__ void st_relaxed(double *p, double v)
-{
-    asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"((unsigned long long)__double_as_longlong(v))
-                 : "memory");
-}
-
-__device__ __forceinline__ float ld_relaxed(const float *p)
-{
-    unsigned v;
-    asm volatile("ld.relaxed.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return __uint_as_float(v);
-}
-
-__device__ __forceinline__ void st_relaxed(float *p, float v)
-{
-    asm volatile("st.relaxed.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(__float_as_uint(v)) : "memory");
-}
-
-__device__ __forceinline__ bool pending(double v) { return (unsigned long long)__double_as_longlong(v) == kPending; }
-__device__ __forceinline__ bool pending(float v) { return __float_as_uint(v) == kPending32; }
-template <class T>
-__device__ __forceinline__ T pending_value();
-template <>
-__device__ __forceinline__ double pending_value<double>() { return __longlong_as_double((long long)kPending); }
-template <>
-__device__ __forceinline__ float pending_value<float>() { return __uint_as_float(kPending32); }
-// a result that happens to carry the pending pattern is stored as a quiet NaN
-__device__ __forceinline__ double unpend(double v) { return pending(v) ? __longlong_as_double((long long)kQuietNaN) : v; }
-__device__ __forceinline__ float unpend(float v) { return pending(v) ? __uint_as_float(kQuietNaN32) : v; }
-
 // Fills the outputs of the coming sweeps with the pending pattern and resets
 // their ticket counters.  x2 may be null.
 template <class T>
@@ -263,29 +224,6 @@ __global__ void k_sweep_prep(int n, T *x1, T *x2, unsigned *t1, unsigned *t2, co
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         x1[i] = p;
         if (x2) x2[i] = p;
-    }
-}
-
-// x_c for a row of the sweep: a relaxed load, polled while it is pending.
-// Gives up (bad) after kSweepSpinLimit polls or when another wait has given
-// up (the context's error flag is set).
-template <class T>
-__device__ __forceinline__ T wait_x(const T *x, int c, const int *err, int spin, bool &bad)
-{
-    T v = ld_relaxed(x + c);
-    if (!pending(v)) return v;
-    unsigned ns = 32;
-    for (long long polls = 1;; ++polls) {
-        if (polls > spin) {
-            __nanosleep(ns);
-            ns = ns < 256 ? 2 * ns : ns;
-        }
-        v = ld_relaxed(x + c);
-        if (!pending(v)) return v;
-        if (polls > kSweepSpinLimit || ((polls & 31) == 0 && *(volatile const int *)err)) {
-            bad = true;
-            return T(0);
-        }
     }
 }
 
@@ -579,6 +517,26 @@ static int build_levels(mtjg_ctx *ctx, int n, int desc, int range, const int *rp
     return MTJG_OK;
 }
 
+static TriOp lower_op(const mtjg_precond *M) { return TriOp{0, M->n, 0, 1, M->rowptr, M->colind, M->diag}; }
+static TriOp upper_op(const mtjg_precond *M) { return TriOp{1, M->n, 1, 2, M->rowptr, M->colind, M->diag}; }
+
+// The schedules of an apply's two sweeps: tiles of lines where the rows form
+// them (lines.cu; `plan`: one of the same factor to use), else the dependency
+// levels of each.
+static int build_sweeps(mtjg_ctx *ctx, const TriOp &a, const double *va, const TriOp &b, const double *vb,
+                        const double *diagv, TilePlan *plan, TilePair *&tile, LevelSchedule &la, LevelSchedule &lb)
+{
+    free_sched(la);
+    free_sched(lb);
+    int st = tile_pair(ctx, a, b, plan, &tile);
+    if (st == MTJG_OK && tile) {
+        st = tile_values(ctx, tile, 0, a, va, diagv);
+        return st == MTJG_OK ? tile_values(ctx, tile, 1, b, vb, diagv) : st;
+    }
+    if (st == MTJG_OK) st = build_levels(ctx, a.n, a.desc, a.range, a.rp, a.ci, a.diag, nullptr, la);
+    return st == MTJG_OK ? build_levels(ctx, b.n, b.desc, b.range, b.rp, b.ci, b.diag, nullptr, lb) : st;
+}
+
 // Fills the outputs of the next sweeps (x2 may be null) with kPending and
 // resets their tickets.
 static cudaError_t sweep_prep(mtjg_ctx *ctx, int n, double *x1, double *x2, LevelSchedule *s1, LevelSchedule *s2,
@@ -595,9 +553,9 @@ static cudaError_t sweep_t(mtjg_ctx *ctx, bool strict, const LevelSchedule &s, c
                            const double *v, const int *diag, const double *diagv, const double *b, double *x,
                            const int *status, const double *aux = nullptr, double omega = 0.0)
 {
+    const int spin = env_int("MTJG_SWEEP_SPIN", kSweepSpin, 0, 1 << 20);
     if (s.num_chunks == 0) return cudaSuccess;
     const int warps = ctx->num_sms * env_int("MTJG_SWEEP_WARPS", kSweepWarpsPerSm, 1, 40);
-    const int spin = env_int("MTJG_SWEEP_SPIN", kSweepSpin, 0, 1 << 20);
     const int grid = (std::min(warps, s.num_chunks) + kSweepBlock / 32 - 1) / (kSweepBlock / 32);
     auto go = [&](auto kernel) {
         kernel<<<grid, kSweepBlock, 0, ctx->stream>>>(s.perm, s.chunk, s.num_chunks, rp, ci, v, diag, diagv, b, x,
@@ -635,11 +593,14 @@ static cudaError_t sweep(mtjg_ctx *ctx, int mode, const LevelSchedule &s, const 
 // Two sweeps, b -> y (first operator) -> x (second): y and (when it does not
 // alias b) x are filled in one pass before the first; an x that aliases b is
 // filled between the two.
-static cudaError_t sweep_pair(mtjg_ctx *ctx, int n, int mode1, LevelSchedule &s1, const int *rp1, const int *ci1,
+static cudaError_t sweep_pair(mtjg_ctx *ctx, int n, const TilePair *tile, int mode1, LevelSchedule &s1, const int *rp1, const int *ci1,
                               const double *v1, const int *diag1, const double *diagv1, int mode2, LevelSchedule &s2,
                               const int *rp2, const int *ci2, const double *v2, const int *diag2,
                               const double *diagv2, const double *b, double *y, double *x, const int *status)
 {
+    if (tile)
+        return tile_apply(ctx, tile, ctx->numerics == MTJG_NUMERICS_STRICT, b, x, status,
+                          env_int("MTJG_SWEEP_SPIN", kSweepSpin, 0, 1 << 20));
     const bool alias = x == b;
     cudaError_t e = sweep_prep(ctx, n, y, alias ? nullptr : x, &s1, &s2, status);
     if (e == cudaSuccess) e = sweep(ctx, mode1, s1, rp1, ci1, v1, diag1, diagv1, b, y, status);
@@ -697,11 +658,11 @@ int precond_apply_dev(mtjg_precond *M, const double *b, double *x, const int *st
     }
     case MTJG_PC_ILU:   // L y = b, then U x = y (S/ILU.java:64-70)
     case MTJG_PC_ILUT:  // the same solves on the ILUT factor (S/ILUT.java:111-113)
-        e = sweep_pair(ctx, n, 0, M->lo, M->rowptr, M->colind, M->data, M->diag, nullptr, 1, M->up, M->rowptr,
+        e = sweep_pair(ctx, n, M->tile, 0, M->lo, M->rowptr, M->colind, M->data, M->diag, nullptr, 1, M->up, M->rowptr,
                        M->colind, M->data, M->diag, nullptr, b, M->y, x, status);
         break;
     default:  // ICC: R' y = b, then R x = y (S/ICC.java:67-73)
-        e = sweep_pair(ctx, n, 2, M->lo, M->rt_rowptr, M->rt_colind, M->rt_val, nullptr, M->diagv, 1, M->up,
+        e = sweep_pair(ctx, n, M->tile, 2, M->lo, M->rt_rowptr, M->rt_colind, M->rt_val, nullptr, M->diagv, 1, M->up,
                        M->rowptr, M->colind, M->data, M->diag, nullptr, b, M->y, x, status);
         break;
     }
@@ -739,9 +700,9 @@ template <int MODE>
 static cudaError_t sweep32(mtjg_ctx *ctx, const LevelSchedule &s, const int *rp, const int *ci, const float *v,
                            const int *diag, const float *b, float *x, const int *status)
 {
+    const int spin = env_int("MTJG_SWEEP_SPIN", kSweepSpin, 0, 1 << 20);
     if (s.num_chunks == 0) return cudaSuccess;
     const int warps = ctx->num_sms * env_int("MTJG_SWEEP_WARPS", kSweepWarpsPerSm, 1, 40);
-    const int spin = env_int("MTJG_SWEEP_SPIN", kSweepSpin, 0, 1 << 20);
     const int grid = (std::min(warps, s.num_chunks) + kSweepBlock / 32 - 1) / (kSweepBlock / 32);
     if (sweep_lookahead(MODE, kLookaheadModes32))
         k_trsv_sweep<false, MODE, float, true><<<grid, kSweepBlock, 0, ctx->stream>>>(
@@ -777,6 +738,11 @@ int precond_prepare32(mtjg_precond *M)
         MTJG_CUDA(cudaMalloc(&M->y32, sizeof(float) * (size_t)std::max(1, n)));
         if (M->nnz) k_narrow<<<ctx->num_sms * 8, kBlock, 0, ctx->stream>>>(M->nnz, M->data, M->data32);
         ctx->launches++;
+        if (M->tile) {
+            int st = tile_values(ctx, M->tile, 0, lower_op(M), M->data32, nullptr);
+            if (st == MTJG_OK) st = tile_values(ctx, M->tile, 1, upper_op(M), M->data32, nullptr);
+            if (st != MTJG_OK) return st;
+        }
     }
     MTJG_CUDA(cudaGetLastError());
     M->v32 = M->version;
@@ -805,6 +771,10 @@ int precond_apply32(mtjg_precond *M, const float *b, float *x, const int *status
         e = cudaGetLastError();
         break;
     default: {  // ILU / ILUT: L y = b, then U x = y, on the FP32 factor
+        if (M->tile) {
+            e = tile_apply(ctx, M->tile, false, b, x, status, env_int("MTJG_SWEEP_SPIN", kSweepSpin, 0, 1 << 20));
+            break;
+        }
         const bool alias = x == b;
         k_sweep_prep<float><<<grid_for(ctx, n), kBlock, 0, ctx->stream>>>(n, M->y32, alias ? nullptr : x,
                                                                           M->lo.ticket, M->up.ticket, status);
@@ -840,6 +810,7 @@ struct IluTrans {
     int *lt_rp = nullptr, *lt_ci = nullptr;
     double *lt_v = nullptr;
     LevelSchedule ut, lt;
+    TilePair *tile = nullptr;  // or both by tiles of lines, on the plan of the factor's own sweeps
 };
 
 }  // namespace mtjg
@@ -876,9 +847,11 @@ static void precond_release(mtjg_precond *M)
         cudaFree(t->lt_v);
         free_sched(t->ut);
         free_sched(t->lt);
+        free_tiles_of(t->tile);
         delete t;
         M->trans = nullptr;
     }
+    free_tiles_of(M->tile);
     M->ready = false;
 }
 
@@ -992,9 +965,7 @@ static int ilu_setup(mtjg_precond *M, int *err_row)
         return fail(MTJG_ERR_ZERO_PIVOT, "Zero pivot encountered on row " + std::to_string(e) + " during ILU process");
     }
     // solve schedules: L (rows ascending, lower range), U (descending, upper range)
-    st = build_levels(ctx, n, 0, 1, M->rowptr, M->colind, M->diag, nullptr, M->lo);
-    if (st != MTJG_OK) return st;
-    return build_levels(ctx, n, 1, 2, M->rowptr, M->colind, M->diag, nullptr, M->up);
+    return build_sweeps(ctx, lower_op(M), M->data, upper_op(M), M->data, nullptr, nullptr, M->tile, M->lo, M->up);
 }
 
 static int icc_setup(mtjg_precond *M, mtjg_csr *A, int *err_row)
@@ -1024,9 +995,8 @@ static int icc_setup(mtjg_precond *M, mtjg_csr *A, int *err_row)
         k_gather_diag<<<grid_for(ctx, n), kBlock, 0, ctx->stream>>>(n, M->diag, M->data, M->diagv);
         ctx->launches++;
     }
-    st = build_levels(ctx, n, 0, 0, M->rt_rowptr, M->rt_colind, nullptr, nullptr, M->lo);
-    if (st != MTJG_OK) return st;
-    return build_levels(ctx, n, 1, 2, M->rowptr, M->colind, M->diag, nullptr, M->up);
+    return build_sweeps(ctx, TriOp{2, n, 0, 0, M->rt_rowptr, M->rt_colind, nullptr}, M->rt_val, upper_op(M), M->data,
+                        M->diagv, nullptr, M->tile, M->lo, M->up);
 }
 
 // SSOR.setMatrix (S/SSOR.java:98-113): F.set(A), the diagonal positions;
@@ -1070,9 +1040,7 @@ static int ilut_setup(mtjg_precond *M, mtjg_csr *A, int *err_row)
         MTJG_CUDA(cudaMemcpy(M->data, fv.data(), sizeof(double) * (size_t)nnz, cudaMemcpyHostToDevice));
     }
     if (n) MTJG_CUDA(cudaMemcpy(M->diag, fdiag.data(), sizeof(int) * (size_t)n, cudaMemcpyHostToDevice));
-    st = build_levels(ctx, n, 0, 1, M->rowptr, M->colind, M->diag, nullptr, M->lo);
-    if (st != MTJG_OK) return st;
-    return build_levels(ctx, n, 1, 2, M->rowptr, M->colind, M->diag, nullptr, M->up);
+    return build_sweeps(ctx, lower_op(M), M->data, upper_op(M), M->data, nullptr, nullptr, M->tile, M->lo, M->up);
 }
 
 extern "C" int mtjg_precond_set_ssor(mtjg_precond *M, int reverse, double omega_f, double omega_r)
@@ -1189,9 +1157,9 @@ static int ilu_trans_setup(mtjg_precond *M)
             ctx->launches++;
         }
     }
-    st = build_levels(ctx, M->n, 0, 0, t->ut_rp, t->ut_ci, nullptr, nullptr, t->ut);
-    if (st != MTJG_OK) return st;
-    return build_levels(ctx, M->n, 1, 0, t->lt_rp, t->lt_ci, nullptr, nullptr, t->lt);
+    return build_sweeps(ctx, TriOp{2, M->n, 0, 0, t->ut_rp, t->ut_ci, nullptr}, t->ut_v,
+                        TriOp{3, M->n, 1, 0, t->lt_rp, t->lt_ci, nullptr}, t->lt_v, M->diagv,
+                        M->tile ? M->tile->plan : nullptr, t->tile, t->ut, t->lt);
 }
 
 static bool lu_kind(const mtjg_precond *M) { return M->kind == MTJG_PC_ILU || M->kind == MTJG_PC_ILUT; }
@@ -1210,7 +1178,7 @@ int mtjg::precond_trans_apply_dev(mtjg_precond *M, const double *b, double *x, c
     int st = ilu_trans_setup(M);
     if (st != MTJG_OK) return st;
     IluTrans *t = static_cast<IluTrans *>(M->trans);
-    cudaError_t e = sweep_pair(M->ctx, M->n, 2, t->ut, t->ut_rp, t->ut_ci, t->ut_v, nullptr, M->diagv, 3, t->lt,
+    cudaError_t e = sweep_pair(M->ctx, M->n, t->tile, 2, t->ut, t->ut_rp, t->ut_ci, t->ut_v, nullptr, M->diagv, 3, t->lt,
                                t->lt_rp, t->lt_ci, t->lt_v, nullptr, nullptr, b, M->y, x, status);
     if (e != cudaSuccess) return cuda_fail(e, "ILU transApply");
     return MTJG_OK;
