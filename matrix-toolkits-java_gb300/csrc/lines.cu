@@ -47,10 +47,17 @@ struct LinePipe {
     static constexpr int kLoaders = sizeof(V) == 8 ? 4 : 8;
 };
 
+// A record: kmax entry values, the diagonal and its reciprocal, the codes.
+// The pivots of ILU(0) (MODE 6) take 2 kmax entry values instead.
 template <class V>
 __host__ __device__ constexpr int line_record(int kmax, int lanes)
 {
     return lanes * ((kmax + 2) * (int)sizeof(V) + 16);
+}
+template <class V, int MODE>
+__host__ __device__ constexpr int mode_record(int kmax, int lanes)
+{
+    return MODE == 6 ? lanes * (2 * kmax * (int)sizeof(V) + 16) : line_record<V>(kmax, lanes);
 }
 // Shared memory: the values a lane may read after a step's barrier -- the
 // ring (kRing steps of x), a zero, the entries from other CTAs (kSlots steps)
@@ -68,15 +75,13 @@ __host__ __device__ constexpr int line_slots(int kmax, int lanes)
 {
     return line_zero<V>(lanes) + 16 + LinePipe<V>::kSlots * kmax * lanes * (int)sizeof(V);
 }
-template <class V>
-__host__ __device__ constexpr int line_slot(int kmax, int lanes)
-{
-    return line_record<V>(kmax, lanes) + lanes * (int)sizeof(V);
-}
-template <class V>
+// MODE 6's values are pairs (a pivot and its reciprocal): everything before
+// the slots takes twice the place, and a code counts twice.
+template <class V, int MODE = 0>
 constexpr int line_smem(int kmax, int lanes)
 {
-    return line_slots<V>(kmax, lanes) + LinePipe<V>::kSlots * line_slot<V>(kmax, lanes);
+    return (MODE == 6 ? 2 : 1) * line_slots<V>(kmax, lanes) +
+           LinePipe<V>::kSlots * (mode_record<V, MODE>(kmax, lanes) + lanes * (int)sizeof(V));
 }
 
 // ------------------------------------------------------------ the plan
@@ -151,87 +156,162 @@ __global__ void k_line_tile(int lines, const int *pstart, const int *scan, const
     }
 }
 
-__device__ __forceinline__ int ld_relaxed_int(const int *p)
+// Lines as nodes: row j of line l (counted from its first) takes step
+// off[l] + j, so line l may not start before off[m] + w for each line m that
+// it reads, w the largest of (place of the entry read) - (place of the row)
+// + 1 over its rows.  dep: up to kLineK such (m, w) per line, m = -1 for none;
+// *bad = 1 for a line that reads more.  One warp per line.
+__global__ void k_line_deps(TriOp op, int lines, const int *line_of, const int *first, int2 *dep, int *bad)
 {
-    int v;
-    asm volatile("ld.relaxed.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-
-// Dependency levels, a lane per line (level is -1 before).  A line reads
-// earlier lines only and warps take lines in order from a ticket counter, so
-// every line a lane waits on is its own warp's or a running or finished
-// warp's; the lanes of a warp poll together and each round moves every lane
-// whose row is ready, so lanes may wait on each other.
-__global__ void k_line_levels(TriOp op, int lines, const int *first, int *level, unsigned *ticket, int *err)
-{
-    const int lane = threadIdx.x & 31;
-    for (;;) {
-        unsigned base = 0;
-        if (lane == 0) base = atomicAdd(ticket, 32u);
-        base = __shfl_sync(0xffffffffu, base, 0);
-        if (base >= (unsigned)lines) return;
-        const int l = (int)base + lane;
-        int i = l < lines ? first[l] : 0;
-        const int end = l < lines ? first[l + 1] : 0;
-        int own = -1;  // the level of the line's previous row
-        int c[kLineK], nx[kLineK];
-        auto load = [&](int r, int *cc) {
-            int b = 0, e = 0;
-            if (r < end) tri_range(op, r, b, e);
+    const int l = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+    if (l >= lines) return;
+    const int r0 = first[l], r1 = first[l + 1];
+    int m[kLineK], w[kLineK];
 #pragma unroll
-            for (int k = 0; k < kLineK; ++k) cc[k] = b + k < e ? op.ci[b + k] : -1;
-        };
-        load(i, c);
-        load(i + 1, nx);
-        long long idle = 0;
-        while (__any_sync(0xffffffffu, i < end)) {
-            bool moved = false;
-            if (i < end) {
-                int lv = 0;
-                bool ready = true;
+    for (int k = 0; k < kLineK; ++k) m[k] = -1, w[k] = -0x40000000;
+    int used = 0;
+    bool over = false;
+    for (int base = r0; base < r1; base += 32) {
+        const int i = base + lane;
+        int cl[kLineK], cw[kLineK], b = 0, e = 0;
+        if (i < r1) tri_range(op, i, b, e);
 #pragma unroll
-                for (int k = 0; k < kLineK; ++k) {
-                    if (c[k] < 0) continue;
-                    const int d = c[k] == i - 1 ? own : ld_relaxed_int(level + c[k]);
-                    if (d < 0) ready = false;
-                    lv = max(lv, d + 1);
-                }
-                if (ready) {
-                    asm volatile("st.relaxed.gpu.global.b32 [%0], %1;" ::"l"(level + i), "r"(lv) : "memory");
-                    own = lv;
-                    i += 1;
-                    moved = true;
-#pragma unroll
-                    for (int k = 0; k < kLineK; ++k) c[k] = nx[k];
-                    load(i + 1, nx);
-                }
+        for (int k = 0; k < kLineK; ++k) {
+            cl[k] = -1;
+            if (b + k < e) {
+                const int c = op.ci[b + k], lc = line_of[c];
+                if (lc != l) cl[k] = lc, cw[k] = (c - first[lc]) - (i - r0) + 1;
             }
-            idle = __any_sync(0xffffffffu, moved) ? 0 : idle + 1;
-            if (idle > kLineSpin || ((idle & 1023) == 1023 && *(volatile int *)err)) {
-                if (lane == 0) atomicExch(err, 1);
-                return;
+        }
+        // one line read by any lane at a time
+        for (;;) {
+            int mine = -1;
+#pragma unroll
+            for (int k = kLineK - 1; k >= 0; --k)
+                if (cl[k] >= 0) mine = cl[k];
+            const unsigned any = __ballot_sync(0xffffffffu, mine >= 0);
+            if (!any) break;
+            const int t = __shfl_sync(0xffffffffu, mine, __ffs(any) - 1);
+            int most = -0x40000000;
+#pragma unroll
+            for (int k = 0; k < kLineK; ++k)
+                if (cl[k] == t) most = max(most, cw[k]), cl[k] = -1;
+            most = __reduce_max_sync(0xffffffffu, most);
+            bool found = false;
+#pragma unroll
+            for (int k = 0; k < kLineK; ++k)
+                if (m[k] == t) w[k] = max(w[k], most), found = true;
+            if (!found) {
+                over |= used == kLineK;
+#pragma unroll
+                for (int k = 0; k < kLineK; ++k)
+                    if (k == used) m[k] = t, w[k] = most;
+                ++used;
             }
         }
     }
+    if (lane == 0) {
+        if (over) *bad = 1;
+#pragma unroll
+        for (int k = 0; k < kLineK; ++k) dep[(size_t)l * kLineK + k] = make_int2(m[k], w[k]);
+    }
 }
 
-// each part's lowest and highest level (a line's levels grow along it)
-__global__ void k_part_span(int lines, const int *first, const int *part_of, const int *level, int *lo, int *hi)
+// The lowest offsets, in one block, and each part's first and last step.
+// Plane after plane: a line starts after the plane's line before it (a scan
+// of the maps t -> max(b, t + a)) and after what it reads in earlier planes.
+// Then rounds over all lines until none moves, which cover what the scan left
+// out (a line reading its own plane's lines beyond the one before) and check
+// the rest; a line reads earlier lines only, so the rounds end (*bad = 1 if
+// not within `lines` rounds).  9216 lines in 96 planes: 634 us by rounds
+// alone (415 us by a level search through the L2), 141 with the scans.  Many
+// short planes (more than kScanPlanes) go by rounds.
+constexpr int kOffsetBlock = 1024;
+constexpr int kScanPlanes = 2048;
+__global__ void __launch_bounds__(kOffsetBlock) k_line_offsets(int lines, int planes, const int *pfirst,
+                                                               const int2 *dep, const int *first, const int *part_of,
+                                                               int *off, int *lo, int *hi, int *bad)
 {
-    for (int l = blockIdx.x * blockDim.x + threadIdx.x; l < lines; l += gridDim.x * blockDim.x) {
-        atomicMin(lo + part_of[l], level[first[l]]);
-        atomicMax(hi + part_of[l], level[first[l + 1] - 1]);
+    extern __shared__ int s_off[];
+    __shared__ int s_a[kOffsetBlock / 32], s_b[kOffsetBlock / 32];
+    constexpr int kNone = -0x20000000;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    for (int l = tid; l < lines; l += kOffsetBlock) s_off[l] = 0;
+    __syncthreads();
+    for (int p = 0; p < planes && planes <= kScanPlanes; ++p) {
+        const int l0 = pfirst[p], l1 = pfirst[p + 1];
+        int carry = kNone;  // the offset of the line before the chunk
+        for (int base = l0; base < l1; base += kOffsetBlock) {
+            const int l = base + tid;
+            int A = kNone, B = 0;  // off = max(B, offset of line l - 1 + A)
+            if (l < l1) {
+                const int4 *d = reinterpret_cast<const int4 *>(dep + (size_t)l * kLineK);
+                int4 q[kLineK / 2];
+#pragma unroll
+                for (int k = 0; k < kLineK / 2; ++k) q[k] = __ldg(d + k);
+#pragma unroll
+                for (int k = 0; k < kLineK; ++k) {
+                    const int m = k & 1 ? q[k / 2].z : q[k / 2].x, w = k & 1 ? q[k / 2].w : q[k / 2].y;
+                    if (m >= 0 && m == l - 1 && l > l0) A = w;
+                    else if (m >= 0 && m < l0) B = max(B, s_off[m] + w);
+                }
+            } else {
+                A = 0, B = kNone;  // the identity
+            }
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {  // inclusive scan of the maps, earlier lines first
+                const int pa = __shfl_up_sync(0xffffffffu, A, o), pb = __shfl_up_sync(0xffffffffu, B, o);
+                if (lane >= o) {
+                    B = max(B, pb + A);
+                    A = max(pa + A, kNone);
+                }
+            }
+            if (lane == 31) s_a[warp] = A, s_b[warp] = B;
+            __syncthreads();
+            int t = carry;  // the offset before this warp's first line
+            for (int w = 0; w < warp; ++w) t = max(s_b[w], t + s_a[w]);
+            const int v = max(B, t + A);
+            if (l < l1) s_off[l] = v;
+            __syncthreads();
+            if (base + kOffsetBlock < l1) carry = s_off[base + kOffsetBlock - 1];
+        }
+    }
+    int round = 0;
+    for (;; ++round) {
+        bool moved = false;
+        for (int l = tid; l < lines; l += kOffsetBlock) {
+            const int2 *d = dep + (size_t)l * kLineK;
+            const int was = ((volatile int *)s_off)[l];
+            int v = was;
+#pragma unroll
+            for (int k = 0; k < kLineK; ++k) {
+                const int2 q = __ldg(d + k);
+                if (q.x >= 0) v = max(v, ((volatile int *)s_off)[q.x] + q.y);
+            }
+            if (v != was) {
+                ((volatile int *)s_off)[l] = v;
+                moved = true;
+            }
+        }
+        if (!__syncthreads_or(moved) || round > lines) break;
+    }
+    if (round > lines && tid == 0) *bad = 1;
+    for (int l = tid; l < lines; l += kOffsetBlock) {
+        const int v = s_off[l];
+        off[l] = v;
+        atomicMin(lo + part_of[l], v);
+        atomicMax(hi + part_of[l], v + first[l + 1] - first[l] - 1);
     }
 }
 
 // each row's position, and the row at each position (row is -1 before)
-__global__ void k_line_place(int n, int lanes, const int *line_of, const int *part_of, const int *lane_of,
-                             const int *level, const int *part_min, const int *part_step, int *pos, int *row)
+__global__ void k_line_place(int n, int lanes, const int *line_of, const int *first, const int *part_of,
+                             const int *lane_of, const int *off, const int *part_min, const int *part_step, int *pos,
+                             int *row)
 {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const int l = line_of[i], p = part_of[l];
-        const int at = (part_step[p] + level[i] - part_min[p]) * lanes + lane_of[l];
+        const int at = (part_step[p] + off[l] + (i - first[l]) - part_min[p]) * lanes + lane_of[l];
         pos[i] = at;
         row[at] = i;
     }
@@ -306,6 +386,17 @@ __global__ void k_line_codes(TriOp op, TilePlan tp, unsigned char *rec, int *cur
     }
 }
 
+// Whether a quotient by d may use its reciprocal (else it is kept as 0 and
+// the quotient takes a real division).
+__device__ __forceinline__ bool line_safe(double d)  // 2^-299 <= |d| < 2^300
+{
+    return (((unsigned)__double2hiint(d) >> 20) & 0x7ffu) - 724u <= 598u;
+}
+__device__ __forceinline__ bool line_safe(float d)  // 2^-40 <= |d| < 2^41
+{
+    return ((__float_as_uint(d) >> 23) & 0xffu) - 87u <= 80u;
+}
+
 // The values of every position: entries in the order the sweep adds them,
 // the diagonal and its reciprocal (1 and 1 without a row).  A row with fewer
 // entries is filled up with ones whose product with the zero is -0, which
@@ -327,10 +418,7 @@ __global__ void k_line_values(TriOp op, TilePlan tp, unsigned char *rec, const V
         const V fill = op.mode >= 2 ? V(0) : -V(0);  // modes 2 and 3 subtract
         for (int k = 0; k < K; ++k) rv[k * T + lane] = k < e - b ? v[op.mode == 3 ? e - 1 - k : b + k] : fill;
         rv[K * T + lane] = d;
-        // the reciprocal, or 0 where a quotient by d needs a real division
-        const V m = fabs(d);
-        const bool safe = sizeof(V) == 8 ? m > V(1e-90) && m < V(1e90) : m > V(1e-12) && m < V(1e12);
-        rv[(K + 1) * T + lane] = safe ? V(1) / d : V(0);
+        rv[(K + 1) * T + lane] = line_safe(d) ? V(1) / d : V(0);
     }
 }
 
@@ -438,24 +526,27 @@ __device__ __forceinline__ bool mbar_test_wait(uint64_t *bar, unsigned parity)
 template <bool S, int MODE, int K, int T, class V>
 __global__ void __launch_bounds__(T + 32 * LinePipe<V>::kLoaders + 32, 1)
     k_line_sweep(const unsigned char *__restrict__ rec, const int *__restrict__ part_step,
-                 const int2 *__restrict__ rem, int rem_max, const V *b, V *x, const int *status, int *err, int spin)
+                 const int2 *__restrict__ rem, int rem_max, const V *b, V *x, const int *status, int *err, int spin,
+                 int *pivot0)
 {
     constexpr int D = LinePipe<V>::kSlots, LW = LinePipe<V>::kLoaders;
     constexpr bool kDesc = MODE == 1 || MODE == 3, kDiv = MODE == 1 || MODE == 2;
-    constexpr int kRec = line_record<V>(K, T), kSlot = line_slot<V>(K, T), kBytesB = T * (int)sizeof(V);
+    constexpr int kBytesB = T * (int)sizeof(V), kRec = mode_record<V, MODE>(K, T), kSlot = kRec + kBytesB;
+    constexpr int kArrays = MODE == 6 ? 2 * K : K + 2;  // of a record
+    constexpr int W = MODE == 6 ? 2 : 1;                // words of a value
     extern __shared__ __align__(128) unsigned char sm[];
     __shared__ __align__(8) uint64_t full[D];
     __shared__ volatile int s_done, s_abort;
     if (status && *status != ST_RUNNING) return;
     const int tid = (int)threadIdx.x, lane = tid & 31;
     const int step0 = part_step[blockIdx.x], steps = part_step[blockIdx.x + 1] - step0;
-    unsigned char *slots = sm + line_slots<V>(K, T);
+    unsigned char *slots = sm + W * line_slots<V>(K, T);
     if (tid == 0) {
         for (int i = 0; i < D; ++i) mbar_init(&full[i], 2);
         mbar_fence_init();
         s_done = 0;
         s_abort = 0;
-        *reinterpret_cast<V *>(sm + line_zero<V>(T)) = V(0);
+        for (int w = 0; w < W; ++w) reinterpret_cast<V *>(sm + W * line_zero<V>(T))[w] = V(MODE == 6 ? 1 : 0);
     }
     __syncthreads();
     // step s of the sweep is step plan_step(s) of the plan
@@ -507,10 +598,10 @@ __global__ void __launch_bounds__(T + 32 * LinePipe<V>::kLoaders + 32, 1)
             next = look(s + LW);
             // the lanes read step s - D's entries after its barrier: one step more
             if (!__all_sync(0xffffffffu, slot_free(s + 1))) break;
-            V *xs = reinterpret_cast<V *>(sm + line_remote<V>(K, T, s));
+            V *xs = reinterpret_cast<V *>(sm + W * line_remote<V>(K, T, s));
             bool bad = false;
             for (int q = lane; it.x >= 0;) {
-                xs[it.y] = wait_x(x, it.x, err, spin, bad);
+                for (int w = 0; w < W; ++w) xs[it.y * W + w] = wait_x(x, it.x * W + w, err, spin, bad);
                 q += 32;
                 it = q < rem_max ? rem[(size_t)plan_step(s) * rem_max + q] : make_int2(-1, 0);
             }
@@ -523,16 +614,19 @@ __global__ void __launch_bounds__(T + 32 * LinePipe<V>::kLoaders + 32, 1)
         int slot = 0;         // of the coming step
         unsigned parity = 0;  // of its barrier
         struct Operands {
-            V vv[K], bi, d, y;
+            V vv[K], ww[K], bi, d, y;
             int4 code;
         } even, odd;
         auto fetch = [&](Operands &o, int sl) {
             const unsigned char *at = slots + sl * kSlot;
             const V *cv = reinterpret_cast<const V *>(at) + tid;
-            o.code = reinterpret_cast<const int4 *>(at + (K + 2) * kBytesB)[tid];
+            o.code = reinterpret_cast<const int4 *>(at + kArrays * kBytesB)[tid];
             o.bi = reinterpret_cast<const V *>(at + kRec)[tid];
 #pragma unroll
-            for (int k = 0; k < K; ++k) o.vv[k] = cv[k * T];
+            for (int k = 0; k < K; ++k) {
+                o.vv[k] = cv[k * T];
+                if constexpr (MODE == 6) o.ww[k] = cv[(K + k) * T];
+            }
             if constexpr (kDiv) {
                 o.d = cv[K * T];
                 o.y = cv[(K + 1) * T];
@@ -552,8 +646,8 @@ __global__ void __launch_bounds__(T + 32 * LinePipe<V>::kLoaders + 32, 1)
             if (bad) o.code = make_int4(line_zero<V>(T), line_zero<V>(T), line_zero<V>(T), line_zero<V>(T));
         };
         int prev = 0;  // the slot before it
-        V *out = x + (size_t)plan_step(0) * T + tid;
-        int here = tid * (int)sizeof(V);  // this step's place in the ring
+        V *out = x + ((size_t)plan_step(0) * T + tid) * W;
+        int here = tid * (int)sizeof(V) * W;  // this step's place in the ring
         // Step s on `o`.  The next step's operands are read into `next` while
         // the sum's multiply-adds wait for each other (a straight line, for
         // the compiler to interleave), and again after this step's x is out
@@ -562,9 +656,12 @@ __global__ void __launch_bounds__(T + 32 * LinePipe<V>::kLoaders + 32, 1)
         auto step = [&](int s, Operands &o, Operands &next) {
             asm volatile("bar.sync 1, %0;" ::"n"(T) : "memory");  // step s - 1 is in the ring, step s's slot is read
             const int at[4] = {o.code.x, o.code.y, o.code.z, o.code.w};
-            V xv[K];
+            V xv[K], xr[K];
 #pragma unroll
-            for (int k = 0; k < K; ++k) xv[k] = *reinterpret_cast<const V *>(sm + at[k]);
+            for (int k = 0; k < K; ++k) {
+                xv[k] = *reinterpret_cast<const V *>(sm + at[k] * W);
+                if constexpr (W == 2) xr[k] = reinterpret_cast<const V *>(sm + at[k] * W)[1];
+            }
             const int sl = slot;
             const unsigned par = parity;
             const bool early = mbar_test_wait(&full[sl], par);
@@ -576,14 +673,26 @@ __global__ void __launch_bounds__(T + 32 * LinePipe<V>::kLoaders + 32, 1)
             parity ^= slot == 0 ? 1u : 0u;
             V acc = MODE >= 2 ? o.bi : V(0);
 #pragma unroll
-            for (int k = 0; k < K; ++k) acc = fmac<S>(MODE >= 2 ? -o.vv[k] : o.vv[k], xv[k], acc);
+            for (int k = 0; k < K; ++k) {
+                if constexpr (MODE == 6) {  // a_kk -= (a_ki / d_i) a_ik (FP64 only)
+                    acc = fmac<true>(-line_div<true>(o.vv[k], xv[k], xr[k]), o.ww[k], acc);
+                    if ((unsigned long long)__double_as_longlong(xv[k]) << 1 == 0ull) *pivot0 = 1;
+                } else {
+                    acc = fmac<S>(MODE >= 2 ? -o.vv[k] : o.vv[k], xv[k], acc);
+                }
+            }
             if constexpr (MODE <= 1) acc = o.bi - acc;
             if constexpr (kDiv) acc = line_div<S>(acc, o.d, o.y);
             // (the result of an operation is never the pending pattern, a signalling NaN)
             *reinterpret_cast<V *>(sm + here) = acc;
             st_relaxed(out, acc);
-            out += kDesc ? -T : T;
-            here = here + kBytesB >= kRing * kBytesB ? here + kBytesB - kRing * kBytesB : here + kBytesB;
+            if constexpr (W == 2) {
+                const V r = line_safe(acc) ? V(1) / acc : V(0);
+                reinterpret_cast<V *>(sm + here)[1] = r;
+                st_relaxed(out + 1, r);
+            }
+            out += (kDesc ? -T : T) * W;
+            here = here + W * kBytesB >= kRing * W * kBytesB ? here + W * kBytesB - kRing * W * kBytesB : here + W * kBytesB;
             if (!early && s + 1 < steps) wait_fetch(next, sl, par);
         };
         if (steps > 0) {
@@ -602,10 +711,10 @@ namespace {
 
 template <bool S, int MODE, int K, int T, class V>
 cudaError_t launch_line(mtjg_ctx *ctx, const TilePlan *tp, const TileOp &op, const V *b, V *x, const int *status,
-                        int spin)
+                        int spin, int *pivot0 = nullptr)
 {
     auto k = k_line_sweep<S, MODE, K, T, V>;
-    const int smem = line_smem<V>(K, T);
+    const int smem = line_smem<V, MODE>(K, T);
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg{};
@@ -620,25 +729,26 @@ cudaError_t launch_line(mtjg_ctx *ctx, const TilePlan *tp, const TileOp &op, con
     cfg.numAttrs = 1;
     const unsigned char *rec = sizeof(V) == 8 ? op.rec64 : op.rec32;
     e = cudaLaunchKernelEx(&cfg, k, rec, (const int *)tp->part_step, (const int2 *)op.rem, op.rem_max, b, x, status,
-                           ctx->d_flag, spin);
+                           ctx->d_flag, spin, pivot0);
     if (e == cudaSuccess) ctx->launches++;
     return e;
 }
 
 template <bool S, int MODE, class V>
-cudaError_t launch_k(mtjg_ctx *ctx, const TilePlan *tp, const TileOp &op, const V *b, V *x, const int *status, int spin)
+cudaError_t launch_k(mtjg_ctx *ctx, const TilePlan *tp, const TileOp &op, const V *b, V *x, const int *status, int spin,
+                     int *pivot0 = nullptr)
 {
     const bool wide = tp->lanes == 256;
     switch (tp->kmax) {
     case 2:
-        return wide ? launch_line<S, MODE, 2, 256, V>(ctx, tp, op, b, x, status, spin)
-                    : launch_line<S, MODE, 2, 128, V>(ctx, tp, op, b, x, status, spin);
+        return wide ? launch_line<S, MODE, 2, 256, V>(ctx, tp, op, b, x, status, spin, pivot0)
+                    : launch_line<S, MODE, 2, 128, V>(ctx, tp, op, b, x, status, spin, pivot0);
     case 3:
-        return wide ? launch_line<S, MODE, 3, 256, V>(ctx, tp, op, b, x, status, spin)
-                    : launch_line<S, MODE, 3, 128, V>(ctx, tp, op, b, x, status, spin);
+        return wide ? launch_line<S, MODE, 3, 256, V>(ctx, tp, op, b, x, status, spin, pivot0)
+                    : launch_line<S, MODE, 3, 128, V>(ctx, tp, op, b, x, status, spin, pivot0);
     default:
-        return wide ? launch_line<S, MODE, 4, 256, V>(ctx, tp, op, b, x, status, spin)
-                    : launch_line<S, MODE, 4, 128, V>(ctx, tp, op, b, x, status, spin);
+        return wide ? launch_line<S, MODE, 4, 256, V>(ctx, tp, op, b, x, status, spin, pivot0)
+                    : launch_line<S, MODE, 4, 128, V>(ctx, tp, op, b, x, status, spin, pivot0);
     }
 }
 
@@ -762,9 +872,9 @@ static int tile_plan(mtjg_ctx *ctx, const TriOp &op, const TriOp &up, TilePlan *
     } while (0)
     cudaStream_t q = ctx->stream;
     const int g = grid_rows(ctx, n);
-    LP_CUDA(cudaMalloc(&work, sizeof(int) * (4 * (size_t)n + 2 + 4)));
-    int *start = work, *scan = start + n, *line_of = scan + n + 1, *level = line_of + n, *scalars = level + n;
-    // scalars: longest row, lines of the longest plane, ticket, 1 unless mirrored
+    LP_CUDA(cudaMalloc(&work, sizeof(int) * (3 * (size_t)n + 2 + 4)));
+    int *start = work, *scan = start + n, *line_of = scan + n + 1, *scalars = line_of + n;
+    // scalars: longest row, lines of the longest plane, 1 for lines without offsets, 1 unless mirrored
     LP_CUDA(cudaMemsetAsync(scalars, 0, sizeof(int) * 4, q));
     k_line_start<<<g, kBlock, 0, q>>>(op, start);
     k_mirrored<<<g, kBlock, 0, q>>>(op, up, scalars, scalars + 3);
@@ -778,10 +888,12 @@ static int tile_plan(mtjg_ctx *ctx, const TriOp &op, const TriOp &up, TilePlan *
     LP_CUDA(cudaStreamSynchronize(q));
     tp->kmax = sc[0] == 1 ? 2 : sc[0];
     if (tp->kmax < 2 || tp->kmax > kLineK || sc[3] || (int64_t)lines * kMinLine > n) return done(MTJG_OK, false);
-    // first row of each line, plane starts and their scan, first line of each plane, part and lane
-    LP_CUDA(cudaMalloc(&lw, sizeof(int) * (6 * (size_t)lines + 4)));
-    int *first = lw, *pstart = first + lines + 1, *pscan = pstart + lines, *pfirst = pscan + lines + 1;
-    int *part_of = pfirst + lines + 1, *lane_of = part_of + lines;
+    // what each line reads, first row of each line, plane starts and their
+    // scan, first line of each plane, part, lane and offset
+    LP_CUDA(cudaMalloc(&lw, sizeof(int) * ((7 + 2 * kLineK) * (size_t)lines + 4)));
+    int2 *dep = reinterpret_cast<int2 *>(lw);
+    int *first = lw + 2 * kLineK * (size_t)lines, *pstart = first + lines + 1, *pscan = pstart + lines, *pfirst = pscan + lines + 1;
+    int *part_of = pfirst + lines + 1, *lane_of = part_of + lines, *off = lane_of + lines;
     const int gl = grid_rows(ctx, lines);
     k_line_of<<<g, kBlock, 0, q>>>(n, start, scan, line_of, first, lines);
     k_fill<<<gl, kBlock, 0, q>>>(lines, pstart, 1);
@@ -810,7 +922,7 @@ static int tile_plan(mtjg_ctx *ctx, const TriOp &op, const TriOp &up, TilePlan *
         }
     int optin = 0;
     LP_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
-    if (!tp->parts || line_smem<double>(tp->kmax, tp->lanes) + 1024 > optin ||
+    if (!tp->parts || (int64_t)lines * 4 + 1024 > optin || line_smem<double>(tp->kmax, tp->lanes) + 1024 > optin ||
         line_smem<float>(tp->kmax, tp->lanes) + 1024 > optin)
         return done(MTJG_OK, false);
     const int P = tp->parts, T = tp->lanes;
@@ -818,24 +930,18 @@ static int tile_plan(mtjg_ctx *ctx, const TriOp &op, const TriOp &up, TilePlan *
     LP_CUDA(cudaMalloc(&tp->part_step, sizeof(int) * (size_t)(P + 1)));
     LP_CUDA(cudaMalloc(&tp->pos, sizeof(int) * (size_t)n));
     k_line_tile<<<gl, kBlock, 0, q>>>(lines, pstart, pscan, pfirst, tq, T / tq, ntq, part_of, lane_of);
-    LP_CUDA(cudaMemsetAsync(level, 0xff, sizeof(int) * (size_t)n, q));
-    LP_CUDA(cudaMemsetAsync(ctx->d_flag, 0, sizeof(int), q));
-    const int warps = (lines + 31) / 32;
-    k_line_levels<<<std::max(1, std::min((warps + 3) / 4, ctx->num_sms * 8)), 128, 0, q>>>(
-        op, lines, first, level, reinterpret_cast<unsigned *>(scalars + 2), ctx->d_flag);
     k_fill<<<1, kBlock, 0, q>>>(P, pw, 0x7fffffff);
     k_fill<<<1, kBlock, 0, q>>>(P, pw + P, -1);
-    k_part_span<<<gl, kBlock, 0, q>>>(lines, first, part_of, level, pw, pw + P);
+    k_line_deps<<<(lines + 7) / 8, kBlock, 0, q>>>(op, lines, line_of, first, dep, scalars + 2);
+    LP_CUDA(cudaFuncSetAttribute(k_line_offsets, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - 1024));
+    k_line_offsets<<<1, kOffsetBlock, sizeof(int) * (size_t)lines, q>>>(lines, planes, pfirst, dep, first, part_of, off,
+                                                                        pw, pw + P, scalars + 2);
     ctx->launches += 5;
     std::vector<int> span(2 * (size_t)P), step((size_t)P + 1, 0);
-    int flag = 0;
     LP_CUDA(cudaMemcpyAsync(span.data(), pw, sizeof(int) * 2 * (size_t)P, cudaMemcpyDeviceToHost, q));
-    LP_CUDA(cudaMemcpyAsync(&flag, ctx->d_flag, sizeof(int), cudaMemcpyDeviceToHost, q));
+    LP_CUDA(cudaMemcpyAsync(sc, scalars, sizeof(sc), cudaMemcpyDeviceToHost, q));
     LP_CUDA(cudaStreamSynchronize(q));
-    if (flag) {
-        cudaMemset(ctx->d_flag, 0, sizeof(int));
-        return done(fail(MTJG_ERR_DEVICE_TIMEOUT, "level analysis: a bounded wait gave up"), false);
-    }
+    if (sc[2]) return done(MTJG_OK, false);
     int64_t steps = 0;
     for (int p = 0; p < P; ++p) {
         const int lo = span[(size_t)p], hi = span[(size_t)(P + p)];
@@ -848,7 +954,7 @@ static int tile_plan(mtjg_ctx *ctx, const TriOp &op, const TriOp &up, TilePlan *
     LP_CUDA(cudaMemcpyAsync(tp->part_step, step.data(), sizeof(int) * (size_t)(P + 1), cudaMemcpyHostToDevice, q));
     LP_CUDA(cudaMalloc(&tp->row, sizeof(int) * count));
     LP_CUDA(cudaMemsetAsync(tp->row, 0xff, sizeof(int) * count, q));
-    k_line_place<<<g, kBlock, 0, q>>>(n, T, line_of, part_of, lane_of, level, pw, tp->part_step, tp->pos, tp->row);
+    k_line_place<<<g, kBlock, 0, q>>>(n, T, line_of, first, part_of, lane_of, off, pw, tp->part_step, tp->pos, tp->row);
     ctx->launches++;
     LP_CUDA(cudaMalloc(&tp->b64, sizeof(double) * 3 * count));
     tp->y64 = tp->b64 + count;
@@ -925,6 +1031,111 @@ int tile_pair(mtjg_ctx *ctx, const TriOp &lo, const TriOp &up, TilePlan *plan, T
     if (st != MTJG_OK || !t->plan) free_tiles_of(t);
     else *out = t;
     return st;
+}
+
+// ----------------------------------------------------- ILU(0)'s pivots
+// Where no elimination step finds a column of row k other than k itself
+// (grids without diagonals), ILU.factor (S/ILU.java:98-121) changes only
+// the pivots, in row order: d_k = a_kk - (a_ki / d_i) a_ik over ascending i,
+// and its multipliers are a_ki / d_i.  So the factor is a sweep whose values
+// are the pivots (each with its reciprocal, so that a row takes one division
+// and not one per entry), then one pass over the entries.  96^3 convection-diffusion:
+// 4.2 ms by one launch per level (after 2.4 ms to find the levels), 0.86 ms
+// with a division per entry, 0.41 ms as here; setMatrix and one apply 17.6 ->
+// 3.05 ms, of which about 1 ms allocates and frees.
+//
+// *other = 1 when some step finds another column (MTJ's scan, its read past
+// the row's end included).
+__global__ void k_pivots_only(TriOp lo, int *other)
+{
+    const int *rp = lo.rp, *ci = lo.ci, *diag = lo.diag;
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < lo.n; k += gridDim.x * blockDim.x)
+        for (int i = rp[k]; i < diag[k]; ++i) {
+            const int index = ci[i];
+            for (int j = diag[index] + 1, l = rp[k] + 1; j < rp[index + 1]; ++j) {
+                while (l < rp[k + 1] && ci[l] < ci[j]) l++;
+                if (ci[l] == ci[j] && l != diag[k]) *other = 1;
+            }
+        }
+}
+
+// MODE 6's records, its b (the diagonal) and its output (a pivot and its
+// reciprocal per position) to pending; codes: the records of the lower sweep
+__global__ void k_pivot_records(TriOp lo, TilePlan tp, const unsigned char *codes, const double *data,
+                                unsigned char *rec, double *b, double *x)
+{
+    const int T = tp.lanes, K = tp.kmax, from = line_record<double>(K, T), to = mode_record<double, 6>(K, T);
+    for (int at = blockIdx.x * blockDim.x + threadIdx.x; at < tp.steps * T; at += gridDim.x * blockDim.x) {
+        const int k = tp.row[at], step = at / T, lane = at % T;
+        unsigned char *r = rec + (size_t)step * to;
+        double *rv = reinterpret_cast<double *>(r);
+        reinterpret_cast<int4 *>(r + (size_t)T * 2 * K * sizeof(double))[lane] =
+            reinterpret_cast<const int4 *>(codes + (size_t)step * from + (size_t)T * (K + 2) * sizeof(double))[lane];
+        const int b0 = k >= 0 ? lo.rp[k] : 0, cnt = k >= 0 ? lo.diag[k] - b0 : 0;
+        for (int e = 0; e < K; ++e) {
+            double low = 0.0, up = 0.0;
+            if (e < cnt) {
+                const int i = lo.ci[b0 + e];
+                low = data[b0 + e];
+                for (int j = lo.diag[i] + 1; j < lo.rp[i + 1]; ++j)
+                    if (lo.ci[j] == k) up = data[j];
+            }
+            rv[e * T + lane] = low;
+            rv[(K + e) * T + lane] = up;
+        }
+        b[at] = k >= 0 ? data[lo.diag[k]] : 1.0;
+        x[2 * at] = x[2 * at + 1] = pending_value<double>();
+    }
+}
+
+// the pivots into the diagonal, the multipliers into the lower entries
+__global__ void k_pivots_out(TriOp lo, const int *pos, const double *x, double *data)
+{
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < lo.n; k += gridDim.x * blockDim.x) {
+        data[lo.diag[k]] = x[2 * (size_t)pos[k]];
+        for (int i = lo.rp[k]; i < lo.diag[k]; ++i) data[i] = data[i] / x[2 * (size_t)pos[lo.ci[i]]];
+    }
+}
+
+int tile_ilu(mtjg_ctx *ctx, TilePair *t, const TriOp &lo, double *data, bool *factored)
+{
+    *factored = false;
+    const TilePlan *tp = t->plan;
+    int optin = 0;
+    MTJG_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
+    if (line_smem<double, 6>(tp->kmax, tp->lanes) + 1024 > optin) return MTJG_OK;
+    cudaStream_t q = ctx->stream;
+    const int64_t count = (int64_t)tp->steps * tp->lanes;
+    const size_t bytes = (size_t)tp->steps * mode_record<double, 6>(tp->kmax, tp->lanes);
+    unsigned char *rec = nullptr;
+    MTJG_CUDA(cudaMalloc(&rec, bytes + 16));
+    int *flags = reinterpret_cast<int *>(rec + bytes);  // another column found; zero pivot; the device's error flag
+    int h[3] = {1, 1, 1};
+    cudaError_t e = cudaMemsetAsync(flags, 0, sizeof(int) * 2, q);
+    if (e == cudaSuccess) e = cudaMemsetAsync(ctx->d_flag, 0, sizeof(int), q);
+    k_pivots_only<<<grid_rows(ctx, tp->n), kBlock, 0, q>>>(lo, flags);
+    // (y64 and x64 are one array of twice the positions)
+    k_pivot_records<<<grid_rows(ctx, count), kBlock, 0, q>>>(lo, *tp, t->op[0].rec64, data, rec, tp->b64, tp->y64);
+    ctx->launches += 2;
+    TileOp op = t->op[0];
+    op.rec64 = rec;
+    if (e == cudaSuccess)
+        e = launch_k<false, 6, double>(ctx, tp, op, tp->b64, tp->y64, nullptr, 1 << 20, flags + 1);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(flags + 2, ctx->d_flag, sizeof(int), cudaMemcpyDeviceToDevice, q);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(h, flags, sizeof(h), cudaMemcpyDeviceToHost, q);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(q);
+    cudaFree(rec);
+    if (e != cudaSuccess) return cuda_fail(e, "ILU pivots");
+    if (h[2]) {
+        cudaMemset(ctx->d_flag, 0, sizeof(int));
+        return fail(MTJG_ERR_DEVICE_TIMEOUT, "ILU pivots: a bounded wait gave up");
+    }
+    if (h[0] || h[1]) return MTJG_OK;  // general elimination, which also reports a zero pivot's row
+    k_pivots_out<<<grid_rows(ctx, tp->n), kBlock, 0, q>>>(lo, tp->pos, tp->y64, data);
+    ctx->launches++;
+    MTJG_CUDA(cudaGetLastError());
+    *factored = true;
+    return MTJG_OK;
 }
 
 int tile_values(mtjg_ctx *ctx, TilePair *t, int which, const TriOp &op, const double *v, const double *diagv)

@@ -54,6 +54,10 @@ int tile_pair(mtjg_ctx *ctx, const TriOp &lo, const TriOp &up, TilePlan *plan, T
 // A sweep's values into its records.
 int tile_values(mtjg_ctx *ctx, TilePair *tp, int which, const TriOp &op, const double *v, const double *diagv);
 int tile_values(mtjg_ctx *ctx, TilePair *tp, int which, const TriOp &op, const float *v, const float *diagv);
+// ILU(0) of `data` (the matrix's values, lo its lower triangle) in place,
+// where its elimination changes only the pivots; else *factored is false and
+// data as it was.
+int tile_ilu(mtjg_ctx *ctx, TilePair *tp, const TriOp &lo, double *data, bool *factored);
 void free_tiles_of(TilePair *&tp);
 // x = (second) \ ((first) \ b); x may be b.
 cudaError_t tile_apply(mtjg_ctx *ctx, const TilePair *tp, bool strict, const double *b, double *x, const int *status,

@@ -521,14 +521,15 @@ static TriOp lower_op(const mtjg_precond *M) { return TriOp{0, M->n, 0, 1, M->ro
 static TriOp upper_op(const mtjg_precond *M) { return TriOp{1, M->n, 1, 2, M->rowptr, M->colind, M->diag}; }
 
 // The schedules of an apply's two sweeps: tiles of lines where the rows form
-// them (lines.cu; `plan`: one of the same factor to use), else the dependency
-// levels of each.
+// them (lines.cu; `plan`: one of the same factor to use; `planned`: `tile` is
+// the answer already), else the dependency levels of each.
 static int build_sweeps(mtjg_ctx *ctx, const TriOp &a, const double *va, const TriOp &b, const double *vb,
-                        const double *diagv, TilePlan *plan, TilePair *&tile, LevelSchedule &la, LevelSchedule &lb)
+                        const double *diagv, TilePlan *plan, TilePair *&tile, LevelSchedule &la, LevelSchedule &lb,
+                        bool planned = false)
 {
     free_sched(la);
     free_sched(lb);
-    int st = tile_pair(ctx, a, b, plan, &tile);
+    int st = planned ? MTJG_OK : tile_pair(ctx, a, b, plan, &tile);
     if (st == MTJG_OK && tile) {
         st = tile_values(ctx, tile, 0, a, va, diagv);
         return st == MTJG_OK ? tile_values(ctx, tile, 1, b, vb, diagv) : st;
@@ -930,12 +931,12 @@ static int find_diagonal(mtjg_precond *M, int *err_row)
     return MTJG_OK;
 }
 
-static int ilu_setup(mtjg_precond *M, int *err_row)
+// ILU.factor by dependency levels, one launch per level
+static int ilu_factor_levels(mtjg_precond *M, int *err_row)
 {
     mtjg_ctx *ctx = M->ctx;
     const int n = M->n;
-    int st = find_diagonal(M, err_row);
-    if (st != MTJG_OK) return st;
+    int st = MTJG_OK;
     unsigned char *quirk = nullptr;
     MTJG_CUDA(cudaMalloc(&quirk, (size_t)std::max(1, n)));
     if (n) {
@@ -964,8 +965,23 @@ static int ilu_setup(mtjg_precond *M, int *err_row)
         *err_row = e;
         return fail(MTJG_ERR_ZERO_PIVOT, "Zero pivot encountered on row " + std::to_string(e) + " during ILU process");
     }
+    return MTJG_OK;
+}
+
+static int ilu_setup(mtjg_precond *M, int *err_row)
+{
+    mtjg_ctx *ctx = M->ctx;
+    int st = find_diagonal(M, err_row);
+    if (st != MTJG_OK) return st;
+    // the sweeps' tiles need the pattern alone, and serve the factor where it
+    // changes only pivots
+    st = tile_pair(ctx, lower_op(M), upper_op(M), nullptr, &M->tile);
+    bool factored = false;
+    if (st == MTJG_OK && M->tile) st = tile_ilu(ctx, M->tile, lower_op(M), M->data, &factored);
+    if (st == MTJG_OK && !factored) st = ilu_factor_levels(M, err_row);
+    if (st != MTJG_OK) return st;
     // solve schedules: L (rows ascending, lower range), U (descending, upper range)
-    return build_sweeps(ctx, lower_op(M), M->data, upper_op(M), M->data, nullptr, nullptr, M->tile, M->lo, M->up);
+    return build_sweeps(ctx, lower_op(M), M->data, upper_op(M), M->data, nullptr, nullptr, M->tile, M->lo, M->up, true);
 }
 
 static int icc_setup(mtjg_precond *M, mtjg_csr *A, int *err_row)

@@ -42,6 +42,19 @@ def _ragged(rng):
     return len(keep), np.array(rp, dtype=np.int32), np.array(ci, dtype=np.int32), np.array(v)
 
 
+def _grid9(N, rng):
+    rp, ci, v = [0], [], []
+    for y in range(N):
+        for x in range(N):
+            for dy in (-1, 0, 1):
+                for dx in (-1, 0, 1):
+                    if 0 <= x + dx < N and 0 <= y + dy < N:
+                        ci.append((y + dy) * N + x + dx)
+                        v.append(9.0 if dx == dy == 0 else -1.0 - 0.1 * rng.random())
+            rp.append(len(ci))
+    return N * N, np.array(rp, dtype=np.int32), np.array(ci, dtype=np.int32), np.array(v)
+
+
 def _matrix(name):
     rng = np.random.default_rng(11)
     kind, _, arg = name.partition(":")
@@ -49,6 +62,9 @@ def _matrix(name):
         return _banded(400, [int(t) for t in arg.split(",")], rng)
     if kind == "ragged":
         return _ragged(rng)
+    if kind == "nine":  # 2D nine-point: elimination reaches off the diagonal
+        N = int(arg)
+        return _grid9(N, rng)
     return getattr(workloads, kind)(int(arg))
 
 
@@ -56,7 +72,7 @@ MATRICES = ["poisson2d:4", "poisson2d:33", "poisson2d:130", "poisson3d:5", "pois
             "convdiff3d:36",  # tiles with empty lanes on two sides
             "banded:-1,0,1", "banded:-50,-1,0,1,50",  # one line, and a value further back than the ring
             "banded:-60,-7,-2,-1,0,1,2,7,60",  # four entries a row, two of them in the line
-            "ragged:"]
+            "ragged:", "nine:23"]
 
 
 def _vectors(n):
@@ -71,7 +87,7 @@ def _vectors(n):
 @pytest.mark.parametrize("name", MATRICES)
 def test_apply(ctx, name, kind):
     n, rp, ci, v = _matrix(name)
-    if kind == "icc" and name.startswith(("banded", "ragged")):
+    if kind == "icc" and name.startswith(("banded", "ragged", "nine")):
         v = v.copy()
         rows = np.repeat(np.arange(n), np.diff(rp))
         v[ci != rows] = -1.0  # symmetric
@@ -95,3 +111,19 @@ def test_apply(ctx, name, kind):
                     assert np.max(np.abs(fast - want)) <= 1e-12 * np.max(np.abs(want)), trans
     finally:
         ctx.setNumerics(0)
+
+
+def test_zero_pivot(ctx):
+    """A pivot that elimination makes zero: MTJ's message and row, as the oracle has them."""
+    n, rp, ci, v = workloads.poisson2d(20)
+    v = v.copy()
+    for i in (37, 38):  # d_38 = a_38,38 - (a_38,37 / d_37) a_37,38 - ... made 0 by decoupling row 37 and 38 from above
+        for k in range(rp[i], rp[i + 1]):
+            v[k] = 1.0 if ci[k] in (37, 38) else 0.0
+    A = sparse.CompRowMatrix(n, n, rp, ci, v, ctx)
+    Mo = O.Precond(O.PC_ILU, n)
+    assert Mo.set_matrix(O.Csr(n, n, rp, ci, v)) != 0
+    M = sparse.ILU(A)
+    with pytest.raises(RuntimeError, match="Zero pivot"):
+        M.setMatrix(A)
+    assert M.error_row == Mo.detail
