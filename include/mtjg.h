@@ -358,8 +358,11 @@ MTJG_API int mtjg_solver_set_matrix_monitor(mtjg_solver *S, int enable, double n
  * most 512 product tiles (about 80k rows at 7 entries per row, no row longer
  * than 1152 entries) runs its whole loop in one cooperative launch, the
  * matrix held in shared memory, with the results of the graph path bit for
- * bit; every other solve runs a captured graph of its phase launches.
- * MTJG_LAUNCH_GRAPH: always the graph.  No counterpart in the reference. */
+ * bit; every other solve runs a captured graph of its phase launches, in
+ * which GMRES's Gram-Schmidt takes one cooperative launch per inner step (up
+ * to about 2.4 million rows; the same bits as its phases).
+ * MTJG_LAUNCH_GRAPH: always the graph of phases.  No counterpart in the
+ * reference. */
 enum { MTJG_LAUNCH_AUTO = 0, MTJG_LAUNCH_GRAPH = 1 };
 MTJG_API int mtjg_solver_set_launch(mtjg_solver *S, int mode);
 /* Residual history of the last solve: the (residual, iteration) pairs passed

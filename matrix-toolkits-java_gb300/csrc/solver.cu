@@ -643,6 +643,7 @@ struct GmX {
 }  // namespace mtjg
 
 #include "persist.cuh"
+#include "gmres.cuh"
 
 using namespace mtjg;
 
@@ -710,6 +711,7 @@ struct mtjg_solver {
     double *pc_p2 = nullptr;  // the second p buffer
     unsigned long long *pc_bar = nullptr;
     bool last_persistent = false;
+    unsigned long long *gm_bar = nullptr;  // the one-launch Gram-Schmidt's barrier (gmres.cuh)
     // MatrixIterationMonitor (mtjg_solver_set_matrix_monitor)
     int xmon = 0;
     double normA = 0, normb = 0;
@@ -1027,11 +1029,23 @@ struct Phases {
         double *w = pcm == kPcIdentity ? u : v(V_W);
         // v_0 = r / normr
         PH_CHECK(launch_rows(S->ctx, A->rtiles, GmScale<STRICT>{basis(0), r, S->st, false}, rc(), norm()));
+        // each step's Gram-Schmidt in one launch where the rows fit (gmres.cuh)
+        const OrthPlan<STRICT> orth =
+            S->launch_mode == MTJG_LAUNCH_AUTO && !S->xmon ? orth_plan<STRICT>(S->ctx, A->rtiles) : OrthPlan<STRICT>{};
         for (int i = 0; i < S->restart; ++i) {
             PH_CHECK(launch_spmv(S->ctx, csr(), A->tiles, basis(i), GmAv{u, S->st}, rc(), norm()));
             if (pcm != kPcIdentity) {
                 int st = pc(u, w, &S->st->gate);
                 if (st != MTJG_OK) return st;
+            }
+            if (orth.kernel) {
+                GmOrth a{w, S->V, (size_t)S->n, i, S->M && S->M->kind == MTJG_PC_SSOR, tile_args(A->rtiles), S->gm,
+                         mp(), A->part, S->gm_bar, S->ctx->d_flag};
+                void *args[] = {&a};
+                PH_CHECK(cudaLaunchCooperativeKernel(reinterpret_cast<void *>(orth.kernel), dim3(orth.grid),
+                                                     dim3(kOrthBlock), args, orth.smem, S->ctx->stream));
+                S->ctx->launches++;
+                continue;
             }
             for (int k = 0; k <= i + 1; ++k) {
                 const double *vprev = k > 0 ? basis(k - 1) : nullptr;
@@ -1382,6 +1396,7 @@ int run(mtjg_solver *S, mtjg_csr *A, mtjg_result *res)
     MTJG_CUDA(cudaMemcpyAsync(A->num_running, &S->num_sys, sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
     MTJG_CUDA(cudaMemsetAsync(A->cnt, 0, sizeof(unsigned) * (size_t)ns, ctx->stream));
     MTJG_CUDA(cudaMemsetAsync(ctx->d_flag, 0, sizeof(int), ctx->stream));
+    if (S->gm_bar) MTJG_CUDA(cudaMemsetAsync(S->gm_bar, 0, 3 * sizeof(unsigned long long), ctx->stream));
     // what the loop body needs that allocates: before any capture
     if (needs_transpose(S->kind)) {
         st = csr_ensure_transpose(A);
@@ -1767,6 +1782,7 @@ extern "C" int mtjg_solver_create(mtjg_ctx *ctx, int kind, int n, int restart, m
         ok = ok && cudaMalloc(&S->gm.s, sizeof(double) * ld) == cudaSuccess;
         ok = ok && cudaMalloc(&S->gm.gc, sizeof(double) * ld) == cudaSuccess;
         ok = ok && cudaMalloc(&S->gm.gs, sizeof(double) * ld) == cudaSuccess;
+        ok = ok && cudaMalloc(&S->gm_bar, 3 * sizeof(unsigned long long)) == cudaSuccess;
         if (ok) {
             cudaMemset(S->V, 0, nb * ld);
             cudaMemset(S->gm.H, 0, sizeof(double) * ld * (size_t)restart);
@@ -1800,6 +1816,7 @@ extern "C" int mtjg_solver_destroy(mtjg_solver *S)
     cudaFree(S->gm.s);
     cudaFree(S->gm.gc);
     cudaFree(S->gm.gs);
+    cudaFree(S->gm_bar);
     cudaFree(S->st);
     cudaFree(S->hist_r);
     cudaFree(S->hist_it);
@@ -1893,6 +1910,7 @@ extern "C" int mtjg_solver_set_launch(mtjg_solver *S, int mode)
     if (!S) return fail(MTJG_ERR_ILLEGAL_ARGUMENT, "NULL solver");
     if (mode != MTJG_LAUNCH_AUTO && mode != MTJG_LAUNCH_GRAPH)
         return fail(MTJG_ERR_ILLEGAL_ARGUMENT, "launch mode must be MTJG_LAUNCH_AUTO or MTJG_LAUNCH_GRAPH");
+    if (S->launch_mode != mode) drop_graph(S);
     S->launch_mode = mode;
     return MTJG_OK;
 }
