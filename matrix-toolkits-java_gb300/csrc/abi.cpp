@@ -33,6 +33,11 @@ static void ctx_free(mtjg_ctx *c)
         if (ev) cudaEventDestroy(ev);
     if (c->d_flag) cudaFree(c->d_flag);
     if (c->h_pinned) cudaFreeHost(c->h_pinned);
+    for (cudaStream_t q : c->side)
+        if (q) cudaStreamDestroy(q);
+    for (cudaEvent_t e : c->join)
+        if (e) cudaEventDestroy(e);
+    if (c->fork) cudaEventDestroy(c->fork);
     if (c->stream) cudaStreamDestroy(c->stream);
     delete c;
 }

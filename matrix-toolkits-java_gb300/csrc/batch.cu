@@ -15,6 +15,15 @@
 // by the autotuner below), never on the batch around it or on which CTA
 // takes it: alone and in any batch they are bit-identical.
 //
+// A system of 4096 rows or more is a team of 2, 4 or 8 CTAs (a thread-block
+// cluster): each takes a contiguous share of the rows, partial sums meet in
+// distributed shared memory in rank order, and every CTA runs the scalar
+// steps on its own copy of the state.  One CTA is bound by its SM's FP64
+// pipe (2 multiply-adds a clock: 0.33 ms per iteration of a 50,000-row
+// system of 19 entries a row), so the largest system alone used to set a
+// batch's time.  192 systems of 500 to 50,000 rows, FP64: 30.8 -> 6.8 ms.
+// The team's size follows the system's rows alone, so its results do too.
+//
 // Autotuner: a system class is (rows band, entries-per-row band).  On the
 // first batch that holds a class, short probe solves (kProbeIters
 // iterations on up to kProbeSystems of its systems) are timed with CUDA
@@ -30,6 +39,8 @@
 #include <numeric>
 
 #include "batch.cuh"
+
+#include <cooperative_groups.h>
 
 namespace mtjg {
 
@@ -49,24 +60,71 @@ constexpr unsigned char kPairFlag = 0x80;  // in a system's lanes byte: pair its
 
 namespace {
 
-// Fixed-order block reduction: a fixed butterfly inside each warp, then
-// warps in order by thread 0; the result is broadcast through `out`.
-template <int SLOTS>
-__device__ __forceinline__ void cta_reduce(Acc &a, int type, Acc *warp_acc, Acc &out)
+namespace cg = cooperative_groups;
+
+struct Shared {
+    Acc warp_acc[kBatchBlock / 32];
+    Acc part[2];  // this CTA's partial, in two places by turns
+    Acc out;
+    SysState st;  // the system's state: every CTA of a team keeps the same
+    double sc[4];
+    int status, iter, flag, k;
+};
+
+// A barrier of the team: every write before it is seen after it.
+template <bool TM>
+__device__ __forceinline__ void team_sync()
+{
+    if constexpr (TM) cg::this_cluster().sync();
+    else __syncthreads();
+}
+
+// Fixed-order reduction over the team: a fixed butterfly inside each warp,
+// then warps in order by thread 0, then the team's CTAs in rank order; the
+// result is broadcast through sh.out.
+template <int SLOTS, bool TM>
+__device__ __forceinline__ void team_reduce(Acc &a, int type, Shared &sh, int &turn)
 {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     if constexpr ((SLOTS & kSlotD2) != 0) a.v[2] += (double)a.f[0];
     if constexpr ((SLOTS & kSlotD3) != 0) a.v[3] += (double)a.f[1];
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) acc_shfl_down<SLOTS>(a, off, type);
-    if (lane == 0) warp_acc[w] = a;
+    if (lane == 0) sh.warp_acc[w] = a;
     __syncthreads();
     if (threadIdx.x == 0) {
-        Acc s = warp_acc[0];
-        for (int k = 1; k < kBatchBlock / 32; ++k) acc_merge_m<SLOTS>(s, warp_acc[k], type);
-        out = s;
+        Acc s = sh.warp_acc[0];
+        for (int k = 1; k < kBatchBlock / 32; ++k) acc_merge_m<SLOTS>(s, sh.warp_acc[k], type);
+        if constexpr (TM) sh.part[turn] = s;
+        else sh.out = s;
+    }
+    if constexpr (TM) {
+        team_sync<TM>();
+        if (threadIdx.x == 0) {
+            cg::cluster_group team = cg::this_cluster();
+            Acc s = *team.map_shared_rank(&sh.part[turn], 0);
+            for (int r = 1; r < (int)team.num_blocks(); ++r)
+                acc_merge_m<SLOTS>(s, *team.map_shared_rank(&sh.part[turn], r), type);
+            sh.out = s;
+        }
+        turn ^= 1;
     }
     __syncthreads();
+}
+
+// The rows of a team's CTA: contiguous shares, multiples of a warp's rows.
+template <bool TM>
+__device__ __forceinline__ void team_rows(const BatchCg &a, int sys, int &r0, int &r1)
+{
+    r0 = a.sys_rows[sys];
+    r1 = a.sys_rows[sys + 1];
+    if constexpr (TM) {
+        const int C = (int)cg::this_cluster().num_blocks(), rank = (int)cg::this_cluster().block_rank();
+        const int len = ((r1 - r0 + C - 1) / C + 31) / 32 * 32;
+        const int s0 = min(r1, r0 + rank * len);
+        r1 = min(r1, s0 + len);
+        r0 = s0;
+    }
 }
 
 // row i of A (x gathered), summed by VEC lanes in entry order per lane and a
@@ -137,25 +195,23 @@ __device__ __forceinline__ void row_dot2(const int *__restrict__ rp, const int *
 constexpr int kU = MTJG_BATCH_U;
 constexpr int kU2 = kU > 2 ? 2 : kU;  // the FP64 update loop, whose rows carry five doubles
 
+// the monitor on the CTA's copy of the state; the team's first CTA records
+template <bool TM>
 __device__ __forceinline__ int batch_check(const BatchCg &a, SysState &t, int sys, double r)
 {
     const size_t h = (size_t)sys * a.mon.hist_cap;
-    return monitor_check(t, a.mon, r, a.hist_r + h, a.hist_it + h);
+    MonCfgDev mon = a.mon;
+    if (TM && cg::this_cluster().block_rank() != 0) mon.hist_cap = 0;
+    return monitor_check(t, mon, r, a.hist_r + h, a.hist_it + h);
 }
-
-struct Shared {
-    Acc warp_acc[kBatchBlock / 32];
-    Acc out;
-    double sc[4];
-    int status, iter, flag, k;
-};
 
 // CG + identity / Jacobi on rows [r0, r1): CgInit, then CgP, CgQ, CgUpd per
 // iteration (solver.cu), in one CTA
-template <int VEC, bool S>
-__device__ void cg_system(const BatchCg &a, int sys, Shared &sh)
+template <int VEC, bool S, bool TM>
+__device__ void cg_system(const BatchCg &a, int sys, Shared &sh, int &turn)
 {
-    const int r0 = a.sys_rows[sys], r1 = a.sys_rows[sys + 1];
+    int r0, r1;
+    team_rows<TM>(a, sys, r0, r1);
     const int tid = threadIdx.x, g = tid / VEC, l = tid % VEC;
     constexpr int RPS = kBatchBlock / VEC;
     const int nt = a.mon.norm;
@@ -186,11 +242,11 @@ __device__ void cg_system(const BatchCg &a, int sys, Shared &sh)
             }
         }
     }
-    cta_reduce<kSlotNorm | kSlotD2>(acc, nt, sh.warp_acc, sh.out);
+    team_reduce<kSlotNorm | kSlotD2, TM>(acc, nt, sh, turn);
     if (tid == 0) {
-        SysState &t = a.st[sys];
+        SysState &t = sh.st;
         t.iter = 0;
-        const int c = batch_check(a, t, sys, norm_finish(sh.out.v, nt));
+        const int c = batch_check<TM>(a, t, sys, norm_finish(sh.out.v, nt));
         if (c == ST_RUNNING) t.rho = sh.out.v[2];
         t.status = c;
         sh.status = c;
@@ -215,7 +271,7 @@ __device__ void cg_system(const BatchCg &a, int sys, Shared &sh)
                 if (i < r1) p[i] = first ? zv[u] : fmac<S>(pv[u], beta, zv[u]);
             }
         }
-        __syncthreads();
+        team_sync<TM>();
         acc_zero(acc);
         for (int base = r0; base < r1; base += 2 * RPS) {  // q = A p; p.q
             double dv[2];
@@ -231,9 +287,9 @@ __device__ void cg_system(const BatchCg &a, int sys, Shared &sh)
                 }
             }
         }
-        cta_reduce<kSlotD2>(acc, nt, sh.warp_acc, sh.out);
+        team_reduce<kSlotD2, TM>(acc, nt, sh, turn);
         if (tid == 0) {
-            SysState &t = a.st[sys];
+            SysState &t = sh.st;
             t.alpha = t.rho / sh.out.v[2];
             sh.sc[0] = t.alpha;
         }
@@ -272,12 +328,12 @@ __device__ void cg_system(const BatchCg &a, int sys, Shared &sh)
                 }
             }
         }
-        cta_reduce<kSlotNorm | kSlotD2>(acc, nt, sh.warp_acc, sh.out);
+        team_reduce<kSlotNorm | kSlotD2, TM>(acc, nt, sh, turn);
         if (tid == 0) {
-            SysState &t = a.st[sys];
+            SysState &t = sh.st;
             t.rho_1 = t.rho;
             t.iter++;
-            const int c = batch_check(a, t, sys, norm_finish(sh.out.v, nt));
+            const int c = batch_check<TM>(a, t, sys, norm_finish(sh.out.v, nt));
             if (c == ST_RUNNING) {
                 t.rho = sh.out.v[2];
                 t.beta = t.rho / t.rho_1;
@@ -293,11 +349,12 @@ __device__ void cg_system(const BatchCg &a, int sys, Shared &sh)
 
 // Mixed precision on rows [r0, r1): the outer step and inner FP32 CG of
 // phases.cuh (MxX, MxOuter, MxP, MxQ, MxUpd), in one CTA
-template <int VEC, bool S>
-__device__ void mixed_system(const BatchCg &a, int sys, Shared &sh)
+template <int VEC, bool S, bool TM>
+__device__ void mixed_system(const BatchCg &a, int sys, Shared &sh, int &turn)
 {
     const bool pair = (a.vec[sys] & kPairFlag) != 0;
-    const int r0 = a.sys_rows[sys], r1 = a.sys_rows[sys + 1];
+    int r0, r1;
+    team_rows<TM>(a, sys, r0, r1);
     const int tid = threadIdx.x, g = tid / VEC, l = tid % VEC;
     constexpr int RPS = kBatchBlock / VEC;
     const int nt = a.mon.norm;
@@ -308,7 +365,7 @@ __device__ void mixed_system(const BatchCg &a, int sys, Shared &sh)
     double *x = a.x;
     for (;;) {
         // the outer step: x += d when a correction is pending (MxX) ...
-        if (tid == 0) sh.flag = a.st[sys].pending;
+        if (tid == 0) sh.flag = sh.st.pending;
         __syncthreads();
         const bool pend = sh.flag != 0;
         __syncthreads();  // every thread has read the flag before it is rewritten
@@ -328,9 +385,9 @@ __device__ void mixed_system(const BatchCg &a, int sys, Shared &sh)
                     if (i < r1) x[i] = xv[u] + (double)dv[u];
                 }
             }
-            __syncthreads();
+            team_sync<TM>();
             if (tid == 0) {
-                SysState &t = a.st[sys];
+                SysState &t = sh.st;
                 t.pending = 0;
                 t.iter++;
             }
@@ -361,10 +418,10 @@ __device__ void mixed_system(const BatchCg &a, int sys, Shared &sh)
                 }
             }
         }
-        cta_reduce<kSlotNorm | kSlotD2 | kSlotD3>(acc, nt, sh.warp_acc, sh.out);
+        team_reduce<kSlotNorm | kSlotD2 | kSlotD3, TM>(acc, nt, sh, turn);
         if (tid == 0) {
-            SysState &t = a.st[sys];
-            const int c = batch_check(a, t, sys, norm_finish(sh.out.v, nt));
+            SysState &t = sh.st;
+            const int c = batch_check<TM>(a, t, sys, norm_finish(sh.out.v, nt));
             if (c == ST_RUNNING) {
                 t.phase = 1;
                 t.pending = 1;
@@ -381,7 +438,7 @@ __device__ void mixed_system(const BatchCg &a, int sys, Shared &sh)
         // inner FP32 CG until its stopping test ends the refinement step
         for (;;) {
             if (tid == 0) {
-                const SysState &t = a.st[sys];
+                const SysState &t = sh.st;
                 sh.flag = t.in_fresh;
                 sh.sc[1] = t.in_beta;
             }
@@ -403,7 +460,7 @@ __device__ void mixed_system(const BatchCg &a, int sys, Shared &sh)
                     if (i < r1) p[i] = fresh ? zv[u] : fmaf(pv[u], beta, zv[u]);
                 }
             }
-            __syncthreads();
+            team_sync<TM>();
             acc_zero(acc);
             for (int base = r0; base < r1; base += 2 * RPS) {  // q = A32 p; p.q
                 float dv[2];
@@ -418,9 +475,9 @@ __device__ void mixed_system(const BatchCg &a, int sys, Shared &sh)
                     }
                 }
             }
-            cta_reduce<kSlotD2>(acc, nt, sh.warp_acc, sh.out);
+            team_reduce<kSlotD2, TM>(acc, nt, sh, turn);
             if (tid == 0) {
-                SysState &t = a.st[sys];
+                SysState &t = sh.st;
                 t.in_alpha = t.in_rho / sh.out.v[2];
                 sh.sc[0] = t.in_alpha;
             }
@@ -455,9 +512,9 @@ __device__ void mixed_system(const BatchCg &a, int sys, Shared &sh)
                     acc.f[1] = fmaf(rf, rf, acc.f[1]);
                 }
             }
-            cta_reduce<kSlotD2 | kSlotD3>(acc, nt, sh.warp_acc, sh.out);
+            team_reduce<kSlotD2 | kSlotD3, TM>(acc, nt, sh, turn);
             if (tid == 0) {
-                SysState &t = a.st[sys];
+                SysState &t = sh.st;
                 t.in_iter++;
                 t.in_total++;
                 t.in_fresh = 0;
@@ -480,50 +537,108 @@ __device__ void mixed_system(const BatchCg &a, int sys, Shared &sh)
     }
 }
 
-template <bool S, bool MIXED>
+// Teams of one size take the systems order[0 .. count) of that size.
+template <bool S, bool MIXED, bool TM>
 __global__ void __launch_bounds__(kBatchBlock, kBatchMinBlocks) k_batch_cg(BatchCg a)
 {
     __shared__ Shared sh;
+    int turn = 0, rank = 0;
+    if constexpr (TM) rank = (int)cg::this_cluster().block_rank();
     for (;;) {
-        if (threadIdx.x == 0) sh.k = (int)atomicAdd(a.ticket, 1u);
-        __syncthreads();
-        const int k = sh.k;
-        __syncthreads();
+        if (threadIdx.x == 0 && rank == 0) sh.k = (int)atomicAdd(a.ticket, 1u);
+        team_sync<TM>();
+        int k = sh.k;
+        if constexpr (TM) k = *cg::this_cluster().map_shared_rank(&sh.k, 0);
+        team_sync<TM>();
         if (k >= a.count) return;
         const int sys = a.order[k];
         const int vec = S ? 1 : (a.vec[sys] & ~kPairFlag);
+        if (threadIdx.x == 0) sh.st = a.st[sys];
+        __syncthreads();
         if constexpr (MIXED) {
             switch (vec) {
-            case 2: mixed_system<2, S>(a, sys, sh); break;
-            case 4: mixed_system<4, S>(a, sys, sh); break;
-            case 8: mixed_system<8, S>(a, sys, sh); break;
-            case 32: mixed_system<32, S>(a, sys, sh); break;
-            default: mixed_system<1, S>(a, sys, sh); break;
+            case 2: mixed_system<2, S, TM>(a, sys, sh, turn); break;
+            case 4: mixed_system<4, S, TM>(a, sys, sh, turn); break;
+            case 8: mixed_system<8, S, TM>(a, sys, sh, turn); break;
+            case 32: mixed_system<32, S, TM>(a, sys, sh, turn); break;
+            default: mixed_system<1, S, TM>(a, sys, sh, turn); break;
             }
         } else {
             switch (vec) {
-            case 2: cg_system<2, S>(a, sys, sh); break;
-            case 4: cg_system<4, S>(a, sys, sh); break;
-            case 8: cg_system<8, S>(a, sys, sh); break;
-            case 32: cg_system<32, S>(a, sys, sh); break;
-            default: cg_system<1, S>(a, sys, sh); break;
+            case 2: cg_system<2, S, TM>(a, sys, sh, turn); break;
+            case 4: cg_system<4, S, TM>(a, sys, sh, turn); break;
+            case 8: cg_system<8, S, TM>(a, sys, sh, turn); break;
+            case 32: cg_system<32, S, TM>(a, sys, sh, turn); break;
+            default: cg_system<1, S, TM>(a, sys, sh, turn); break;
             }
         }
         __syncthreads();
+        if (threadIdx.x == 0 && rank == 0) a.st[sys] = sh.st;
     }
 }
 
+// One launch for the teams of `team` CTAs, on `stream`.
 template <bool S, bool MIXED>
-cudaError_t launch_one(mtjg_ctx *ctx, const BatchCg &a)
+cudaError_t launch_teams(mtjg_ctx *ctx, const BatchCg &a, int team, cudaStream_t stream)
 {
-    auto k = k_batch_cg<S, MIXED>;
+    auto k = team > 1 ? k_batch_cg<S, MIXED, true> : k_batch_cg<S, MIXED, false>;
     int per_sm = 0;
     cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kBatchBlock, 0);
     if (e != cudaSuccess) return e;
-    const int grid = std::max(1, std::min(a.count, ctx->num_sms * std::max(1, per_sm)));
-    k<<<grid, kBatchBlock, 0, ctx->stream>>>(a);
-    ctx->launches++;
-    return cudaGetLastError();
+    const int64_t room = std::max(team, ctx->num_sms * std::max(1, per_sm) / team * team);
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)std::max<int64_t>(1, std::min<int64_t>((int64_t)a.count * team, room)));
+    cfg.blockDim = dim3(kBatchBlock);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = (unsigned)team;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = team > 1 ? 1 : 0;
+    e = cudaLaunchKernelEx(&cfg, k, a);
+    if (e == cudaSuccess) ctx->launches++;
+    return e;
+}
+
+template <bool S, bool MIXED>
+cudaError_t launch_one(mtjg_ctx *ctx, BatchCg a, const int *counts)
+{
+    // each size of team on a stream of its own, between two events of the
+    // context's stream; the largest first
+    int sizes = 0;
+    for (int c = 0; c < kTeamSizes; ++c) sizes += counts[c] > 0;
+    cudaError_t e = cudaSuccess;
+    if (sizes > 1) {
+        for (int c = 0; c + 1 < kTeamSizes && e == cudaSuccess; ++c) {
+            if (!ctx->side[c]) e = cudaStreamCreateWithFlags(&ctx->side[c], cudaStreamNonBlocking);
+            if (e == cudaSuccess && !ctx->join[c]) e = cudaEventCreateWithFlags(&ctx->join[c], cudaEventDisableTiming);
+        }
+        if (e == cudaSuccess && !ctx->fork) e = cudaEventCreateWithFlags(&ctx->fork, cudaEventDisableTiming);
+        if (e == cudaSuccess) e = cudaEventRecord(ctx->fork, ctx->stream);
+    }
+    bool forked[kTeamSizes] = {};
+    int left = sizes;
+    for (int c = 0; c < kTeamSizes && e == cudaSuccess; ++c) {
+        if (counts[c] > 0) {
+            BatchCg b = a;
+            b.count = counts[c];
+            b.ticket = a.ticket + c;
+            // the last size stays on the context's stream
+            const bool side = --left > 0;
+            if (side) e = cudaStreamWaitEvent(ctx->side[c], ctx->fork, 0);
+            if (e == cudaSuccess) e = launch_teams<S, MIXED>(ctx, b, 1 << (kTeamSizes - 1 - c), side ? ctx->side[c] : ctx->stream);
+            if (e == cudaSuccess && side) e = cudaEventRecord(ctx->join[c], ctx->side[c]);
+            forked[c] = side && e == cudaSuccess;
+        }
+        a.order += counts[c];
+    }
+    for (int c = 0; c < kTeamSizes; ++c)
+        if (forked[c]) {
+            const cudaError_t w = cudaStreamWaitEvent(ctx->stream, ctx->join[c], 0);
+            if (e == cudaSuccess) e = w;
+        }
+    return e;
 }
 
 // ----------------------------------------------------------- autotuner
@@ -539,11 +654,27 @@ int band(double v, const double *edges, int count)
 
 }  // namespace
 
-cudaError_t batch_launch(mtjg_ctx *ctx, const BatchCg &a, bool mixed)
+// CTAs of a system's team, as log2.  A share of 2048 rows or more is worth
+// the team's three barriers and rank-order sums per iteration (about 6000
+// cycles against 27,000 of FP64 work for 2048 rows of 19 entries).
+int batch_team(int64_t rows) { return rows >= 16384 ? 3 : rows >= 8192 ? 2 : rows >= 4096 ? 1 : 0; }
+
+void batch_teams(const int *sys_rows, std::vector<int> &order, int *counts)
+{
+    std::vector<int> by[kTeamSizes];
+    for (int s : order) by[kTeamSizes - 1 - batch_team((int64_t)sys_rows[s + 1] - sys_rows[s])].push_back(s);
+    order.clear();
+    for (int c = 0; c < kTeamSizes; ++c) {
+        counts[c] = (int)by[c].size();
+        order.insert(order.end(), by[c].begin(), by[c].end());
+    }
+}
+
+cudaError_t batch_launch(mtjg_ctx *ctx, const BatchCg &a, const int *counts, bool mixed)
 {
     const bool strict = ctx->numerics == MTJG_NUMERICS_STRICT;
-    if (strict) return mixed ? launch_one<true, true>(ctx, a) : launch_one<true, false>(ctx, a);
-    return mixed ? launch_one<false, true>(ctx, a) : launch_one<false, false>(ctx, a);
+    if (strict) return mixed ? launch_one<true, true>(ctx, a, counts) : launch_one<true, false>(ctx, a, counts);
+    return mixed ? launch_one<false, true>(ctx, a, counts) : launch_one<false, false>(ctx, a, counts);
 }
 
 // The class of a system: bands of its rows and of its entries per row.

@@ -18,7 +18,7 @@ struct BatchCg {
     const int *order;           // [count]: the systems, in the order CTAs take them
     const unsigned char *vec;   // [num_sys]: lanes per row
     unsigned *ticket;           // zero at launch
-    int count;
+    int count;                  // systems of this launch's team size
     int pc;                     // kPcIdentity or kPcJacobi
     const double *invdiag;
     const float *invdiag32;
@@ -32,7 +32,13 @@ struct BatchCg {
     MixCfg mix;
 };
 
-cudaError_t batch_launch(mtjg_ctx *ctx, const BatchCg &a, bool mixed);
+constexpr int kTeamSizes = 4;  // teams of 8, 4, 2 and 1 CTAs
+// Puts the systems of each team size together, largest teams first, each
+// keeping its order; counts[c]: systems of teams of 8 >> c CTAs.
+void batch_teams(const int *sys_rows, std::vector<int> &order, int *counts);
+// a.order as batch_teams left it (a.count is not read); a.ticket: kTeamSizes
+// counters, zero.
+cudaError_t batch_launch(mtjg_ctx *ctx, const BatchCg &a, const int *counts, bool mixed);
 int batch_class(int64_t rows, int64_t nnz);
 int batch_tuned(int cls);
 // Lanes per row of each system (tuned per class, probing classes not seen

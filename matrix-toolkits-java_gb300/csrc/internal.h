@@ -218,6 +218,10 @@ struct mtjg_ctx {
     std::atomic<int64_t> launches{0};  // kernels launched (a serving thread counts here too)
     int *d_flag = nullptr;          // device error flag (bounded waits)
     int *h_pinned = nullptr;        // pinned host words for status polling
+    // batched solves run each size of team beside the others (batch.cu);
+    // made on first use, ordered on both sides with `stream`
+    cudaStream_t side[3] = {};
+    cudaEvent_t fork = nullptr, join[3] = {};
 };
 
 struct mtjg_csr {

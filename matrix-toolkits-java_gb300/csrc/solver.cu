@@ -1525,7 +1525,7 @@ int run_batch(mtjg_solver *S, mtjg_csr *A, mtjg_result *res)
         MTJG_CUDA(cudaMalloc(&S->b_vec, (size_t)ns));
         S->b_cap = ns;
     }
-    if (!S->b_ticket) MTJG_CUDA(cudaMalloc(&S->b_ticket, sizeof(unsigned)));
+    if (!S->b_ticket) MTJG_CUDA(cudaMalloc(&S->b_ticket, sizeof(unsigned) * kTeamSizes));
     const int *srow = A->sys_rows.data();
     const int *hrp = A->h_rowptr.data();
     // the systems' row offsets on the device, uploaded once per matrix
@@ -1569,11 +1569,13 @@ int run_batch(mtjg_solver *S, mtjg_csr *A, mtjg_result *res)
         return cudaMemcpyAsync(S->st, S->last_all.data(), sizeof(SysState) * (size_t)ns, cudaMemcpyHostToDevice,
                                ctx->stream);
     };
-    auto go = [&](const BatchCg &args, const std::vector<int> &order) -> cudaError_t {
+    auto go = [&](const BatchCg &args, std::vector<int> order) -> cudaError_t {
+        int counts[kTeamSizes];
+        batch_teams(srow, order, counts);
         cudaError_t e = cudaMemcpyAsync(S->b_order, order.data(), sizeof(int) * order.size(), cudaMemcpyHostToDevice,
                                         ctx->stream);
-        if (e == cudaSuccess) e = cudaMemsetAsync(S->b_ticket, 0, sizeof(unsigned), ctx->stream);
-        if (e == cudaSuccess) e = batch_launch(ctx, args, S->mixed);
+        if (e == cudaSuccess) e = cudaMemsetAsync(S->b_ticket, 0, sizeof(unsigned) * kTeamSizes, ctx->stream);
+        if (e == cudaSuccess) e = batch_launch(ctx, args, counts, S->mixed);
         return e;
     };
     // lanes per row: STRICT sums every row in entry order (one lane)
@@ -1602,7 +1604,6 @@ int run_batch(mtjg_solver *S, mtjg_csr *A, mtjg_result *res)
             }
             std::vector<unsigned char> all((size_t)ns, (unsigned char)lanes);
             BatchCg pa = a;
-            pa.count = (int)pick.size();
             pa.mon.hist_cap = 0;
             if (S->mixed) {
                 pa.mon.max_iter = 1;
@@ -1635,7 +1636,6 @@ int run_batch(mtjg_solver *S, mtjg_csr *A, mtjg_result *res)
     std::stable_sort(order.begin(), order.end(), [&](int x, int y) {
         return (int64_t)hrp[srow[x + 1]] - hrp[srow[x]] > (int64_t)hrp[srow[y + 1]] - hrp[srow[y]];
     });
-    a.count = ns;
     MTJG_CUDA(cudaMemcpyAsync(S->b_vec, vec.data(), vec.size(), cudaMemcpyHostToDevice, ctx->stream));
     MTJG_CUDA(upload_states());
     MTJG_CUDA(cudaMemsetAsync(ctx->d_flag, 0, sizeof(int), ctx->stream));
