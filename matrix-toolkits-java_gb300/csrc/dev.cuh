@@ -54,6 +54,13 @@ __device__ __forceinline__ double jmax(double a, double b)
     return a >= b ? a : b;
 }
 
+// Programmatic dependent launch: a phase's kernel may be launched while the
+// one before it still runs (launch_pdl, spmv.cuh); it waits here for that
+// one's end before it reads or writes anything, then lets the next one in,
+// so the launch latency between dependent phases is paid beside the work.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ----------------------------------------------------------- partial sums
 // Acc slots: v[0], v[1] hold a vector norm (ONE/TWO: sum in v[0]; INFINITY:
 // max in v[0]; TWO_ROBUST: (scale, ssq) in v[0], v[1]); v[2], v[3] hold
@@ -236,8 +243,9 @@ __device__ __forceinline__ void group_partial(Acc &a, int group, const RedCtx &r
 
 // System sys's group partials summed in group order by a block of kBlock
 // threads (valid in thread 0): thread t takes groups t, t+B, t+2B, ... with
-// four loads in flight, then the fixed block tree.  Plain loads: a kernel
-// may sum partials that its own blocks wrote before a grid barrier.
+// four loads in flight (sixteen gave 128^3 CG 0.2 % and cost 96^3 BiCGstab
+// 0.6 %), then the fixed block tree.  Plain loads: a kernel may sum partials
+// that its own blocks wrote before a grid barrier.
 template <int SLOTS>
 __device__ __forceinline__ Acc system_sum(const RedCtx &rc, int sys, int type, double *sm)
 {
@@ -309,6 +317,8 @@ __global__ void __launch_bounds__(kBlock) k_finalize(Op op, RedCtx rc, int type)
     constexpr int SLOTS = OpSlots<Op>::value;
     __shared__ double sm[kParts * kBlock];
     const int sys = blockIdx.x;
+    pdl_wait();
+    pdl_trigger();
     if (!op.active(sys)) return;
     if constexpr (XN) xnorm_block(op.m.st[sys], op.m.mon.norm, sm);
     const Acc s = system_sum<SLOTS>(rc, sys, type, sm);
