@@ -5,29 +5,27 @@
 // (p, q = A p, its finalize, the update, its finalize) is a few dependent
 // L2 round trips wide, and the iteration costs their latency plus the launch
 // gaps.  Here one cooperative launch runs the iterations of the same loop
-// (S/CG.java:66-87) until the monitor stops the solve, with three changes of
-// schedule and none of arithmetic:
-//   - each CTA copies its product tiles (row offsets, columns, values) into
-//     shared memory once, so an iteration reads the matrix from there;
-//   - p = z + beta p is formed where the product gathers it (both operands
-//     gathered, the same fused multiply-add), into the other of two p
-//     buffers, so the p phase and its grid barrier go;
-//   - the update loads all of a thread's rows before its first store.
-// Two grid barriers per iteration remain: after the product (alpha needs
-// every p.q partial) and after the update (beta and the monitor's test need
-// every partial of r).  Every CTA then sums the partials itself, in group
-// order with k_finalize's block tree (system_sum), and applies the scalar
-// step to its own copy of the system's state, so every copy holds the same
-// alpha, beta and status; CTA 0 alone writes the residual history, the
-// running count and, at the end, the state.  The tiles, the groups, the
-// per-thread row order and the block trees are the graph path's, so x, the
-// history and the iteration count are the graph path's bit for bit.
+// (S/CG.java:66-87) until the monitor stops the solve.  A CTA owns one or two
+// product tiles: their entries stay in shared memory and its rows' x, r, z, p
+// and inverse diagonal in registers, so an iteration's traffic is p for the
+// other tiles' gathers and the partial sums.  Three exchanges remain: p (once
+// beta is known), the p.q partials (alpha), the partials of r (beta and the
+// monitor's test).  Each travels as 16-byte packets of a value and a tag (the
+// iteration or phase), stored and polled whole (b128), so nothing is fenced:
+// a fence took 1100 to 3900 cycles of an iteration's 24,000, twice.  Every
+// CTA sums the partials itself, in k_finalize's order and block tree, and
+// applies the scalar step to its own copy of the state; CTA 0 alone writes
+// the history, the running count and the state.  The systems that qualify run
+// CG's row phases on their product tiles on the graph path too, so x, the
+// history and the iteration count are the same on both paths bit for bit.
 //
-// Vectors written in the launch are read with plain loads (the read-only
-// path is for data fixed for a kernel's lifetime); the matrix and the
-// inverse diagonal stay on it.  Barrier waits are bounded: a CTA that gives
-// up sets the error flag and the abort word, and every CTA leaves at its
-// next barrier.
+// 2D Poisson 128^2 (392 iterations): 5.44 ms with the vectors in the L2, row
+// tiles of 1024 rows for the update (16 CTAs of 71) and an arrival counter
+// read before the partials; 4.24 ms with fences around plain partials; 3.03
+// ms as here.
+//
+// Waits are bounded: a CTA that gives up sets the error flag and the abort
+// word, and every CTA leaves at its next wait.
 #pragma once
 
 #include "spmv.cuh"
@@ -64,15 +62,12 @@ struct GridBar {
 // What the one-launch CG reads and writes (the solver's vectors and tiles).
 struct PersistCg {
     CsrArgs A;
-    TileArgs pt;  // product tiles (a tile is a group)
-    TileArgs rt;  // row tiles (a tile is a group)
+    TileArgs pt;  // product tiles: groups of the product's and the update's sums
     const double *invdiag;
-    double *x, *r, *z, *q;
-    double *p[2];  // p of the even / odd iterations
+    double *x, *r, *z;
     int pc;
-    int slots;     // product tiles cached per CTA (tile bid + k G in slot k)
-    RedCtx rcq;    // the product's partials (a buffer of their own)
-    RedCtx rcu;    // the update's partials
+    // packets: p of each row [n], and the partials' two sets [2][tiles][3]
+    ulonglong2 *p, *part;
     MonPtrs m;
     GridBar gb;
     int *err;
@@ -122,118 +117,219 @@ __device__ bool grid_barrier(const GridBar &gb, unsigned long long target, int *
     return s_ok != 0;
 }
 
-// p_j of this iteration, formed as CgP forms it: z_j (first) or beta p_j + z_j
-template <bool S>
-__device__ __forceinline__ double p_of(const double *po, const double *z, int j, bool first, double beta)
+// A packet: a value and its tag, written and read as one 128-bit access.
+__device__ __forceinline__ ulonglong2 ld_packet(const ulonglong2 *p)
 {
-    return first ? z[j] : fmac<S>(po[j], beta, z[j]);
+    ulonglong2 v;
+    asm volatile("{\n\t.reg .b128 t;\n\tld.relaxed.gpu.global.b128 t, [%2];\n\tmov.b128 {%0, %1}, t;\n\t}"
+                 : "=l"(v.x), "=l"(v.y)
+                 : "l"(p)
+                 : "memory");
+    return v;
 }
 
-// q = A p over cached tile slot k (tile t) with CgQ's epilogue, in k_spmv's
-// order: one thread per row (STRICT, or a 1-lane tile), else VEC lanes per
-// row with strided entries and a butterfly.  The row's own p_r is stored
-// into pn (by the thread that hands the row to the epilogue).
-template <bool S, int VEC>
-__device__ __forceinline__ void pcg_tile(const PersistCg &c, const CgQ<S> &qop, const unsigned char *slot, int t,
-                                         const double *po, double *pn, bool first, double beta, Acc &acc)
+__device__ __forceinline__ void st_packet(ulonglong2 *p, double v, unsigned long long tag)
 {
-    const double *sv = reinterpret_cast<const double *>(slot);
-    const int *sc = reinterpret_cast<const int *>(slot + kSlotValBytes);
-    const int *sr = reinterpret_cast<const int *>(slot + kSlotValBytes + kSlotColBytes);
-    const double *z = c.z;
-    const int tid = threadIdx.x;
-    const int r0 = c.pt.tile_row[t], r1 = c.pt.tile_row_end[t];
-    if constexpr (VEC == 1) {
-        for (int r = r0 + tid; r < r1; r += kBlock) {
-            const int b = sr[r - r0], e = sr[r - r0 + 1];
-            double sum = qop.init(r, 0);
-#pragma unroll 8
-            for (int k = b; k < e; ++k) sum = fmac<S>(sv[k], p_of<S>(po, z, sc[k], first, beta), sum);
-            const double pr = p_of<S>(po, z, r, first, beta);
-            pn[r] = pr;
-            qop.row(r, 0, sum, pr, acc);
-        }
-    } else {
-        const int gg = tid / VEC, l = tid % VEC;
-        for (int base = r0; base < r1; base += kBlock / VEC) {
-            const int r = base + gg;
-            double sum = 0.0;
-            if (r < r1 && l == 0) sum = qop.init(r, 0);
-            if (r < r1) {
-                const int b = sr[r - r0], e = sr[r - r0 + 1];
-                for (int k = b + l; k < e; k += VEC) sum = fmac<S>(sv[k], p_of<S>(po, z, sc[k], first, beta), sum);
-            }
-#pragma unroll
-            for (int off = VEC / 2; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off, VEC);
-            if (r < r1 && l == 0) {
-                const double pr = p_of<S>(po, z, r, first, beta);
-                pn[r] = pr;
-                qop.row(r, 0, sum, pr, acc);
-            }
-        }
+    asm volatile("{\n\t.reg .b128 t;\n\tmov.b128 t, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], t;\n\t}" ::"l"(p),
+                 "l"((unsigned long long)__double_as_longlong(v)), "l"(tag)
+                 : "memory");
+}
+
+// One more round of waiting: false when the wait has to end (kGridSpinLimit
+// rounds, or another wait gave up): the CTA's s_bad, the abort word and the
+// error flag are set then.
+__device__ __forceinline__ bool wait_on(const PersistCg &c, long long i, int *s_bad)
+{
+    if (i <= kGridSpinLimit && ((i & 255) != 255 || (!*(volatile int *)c.gb.abort && !*(volatile int *)s_bad)))
+        return true;
+    *(volatile int *)s_bad = 1;
+    atomicExch(c.gb.abort, 1);
+    atomicExch(c.err, 1);
+    return false;
+}
+
+// The value of a packet once it carries `tag` (0 when the wait gives up).
+__device__ double wait_packet(const PersistCg &c, const ulonglong2 *p, unsigned long long tag, int *s_bad)
+{
+    ulonglong2 v = ld_packet(p);
+    for (long long i = 0; v.y != tag && wait_on(c, i, s_bad); ++i) v = ld_packet(p);
+    return v.y == tag ? __longlong_as_double((long long)v.x) : 0.0;
+}
+
+// The tiles' partial sums of one phase meet in one of two sets of packets by
+// turns, tagged with the phase.  Collecting a phase's partials waits for every
+// CTA to be that far; a CTA publishes two phases on only after it has seen
+// every partial of the phase between, which each CTA published after it had
+// collected this one's, so no packet is overwritten before all have read it.
+// For the same reason a row's p is overwritten only after every gather of it.
+// Word w (0, 1: the norm, 2: the plain sum) of a tile's partial, a line of its
+// own: every CTA polls every one, and a line that several CTAs write while
+// others poll it is slow (128^2: 4.08 ms with the tiles' words side by side,
+// 3.57 with 48 bytes a tile, 3.03 with 128).
+constexpr int kPacketStride = 8;
+__device__ __forceinline__ ulonglong2 *partial(const PersistCg &c, int phase, int w, int t)
+{
+    return c.part + ((size_t)(phase & 1) * c.pt.num_tiles + t) * kPacketStride + w;
+}
+
+// The kBlock computing threads' barrier (the scalar warp is not in it).
+__device__ __forceinline__ void rows_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kBlock) : "memory"); }
+
+// block_reduce over the computing threads, of which only the first `used`
+// hold anything: the sums of the empty ones are one zero.  The norm by warp
+// 0, the plain sum by warp 1 (each on a quarter of the SM of its own: a
+// dependent FP64 addition takes 64 cycles there, twelve of them a sum);
+// results in out[0..1] (norm) and out[2], seen after the next barrier.
+template <int SLOTS>
+__device__ __forceinline__ void rows_reduce(const Acc &a, int used, int type, double *sm, double *out)
+{
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const bool robust = type == MTJG_NORM_TWO_ROBUST;
+    if constexpr ((SLOTS & kSlotNorm) != 0) {
+        sm[tid] = a.v[0];
+        if (robust) sm[kBlock + tid] = a.v[1];
     }
-}
-
-// Row tile t of the update (CgUpd::rows with plain loads): x += alpha p,
-// r -= alpha q, z = M r, the |r| and r.z partials in row order.
-template <bool S>
-__device__ __forceinline__ void pcg_update(const PersistCg &c, const double *p, int t, double al, int nt, Acc &acc)
-{
-    constexpr int U = kRowsPerThread;
-    const int r0 = c.rt.tile_row[t], r1 = c.rt.tile_row_end[t];
-    const bool jac = c.pc == kPcJacobi;
-    for (int base = r0 + (int)threadIdx.x; base < r1; base += kRowTile) {
-        double rv[U], xv[U], pv[U], qv[U], dv[U];
+    if constexpr ((SLOTS & kSlotD2) != 0) sm[2 * kBlock + tid] = a.v[2];
+    rows_sync();
+    auto plain = [&](const double *v) {
+        double s = v[lane];
+        for (int i = lane + 32; i - lane < used; i += 32) s += v[i];
+        if (used <= kBlock - 32) s += 0.0;
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const int i = base + u * kBlock;
-            const bool in = i < r1;
-            rv[u] = in ? c.r[i] : 0.0;
-            xv[u] = in ? c.x[i] : 0.0;
-            pv[u] = in ? p[i] : 0.0;
-            qv[u] = in ? c.q[i] : 0.0;
-            dv[u] = in && jac ? __ldg(c.invdiag + i) : 0.0;
-        }
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const int i = base + u * kBlock;
-            if (i >= r1) break;
-            double rr = rv[u];
-            if (al != 0) {
-                c.x[i] = fmac<S>(al, pv[u], xv[u]);
-                rr = fmac<S>(-al, qv[u], rr);
-                c.r[i] = rr;
-            }
-            norm_add<S>(acc, rr, nt);
-            if (jac) {
-                const double zz = rr * dv[u];
-                c.z[i] = zz;
-                acc.v[2] = fmac<S>(rr, zz, acc.v[2]);
+        for (int off = 16; off > 0; off >>= 1) s += __shfl_down_sync(0xffffffffu, s, off);
+        return s;
+    };
+    if constexpr ((SLOTS & kSlotNorm) != 0) {
+        if (warp == 0) {
+            if (type == MTJG_NORM_ONE || type == MTJG_NORM_TWO) {
+                const double s = plain(sm);
+                if (lane == 0) out[0] = s, out[1] = 0.0;
             } else {
-                acc.v[2] = fmac<S>(rr, rr, acc.v[2]);
+                Acc s, o;
+                s.v[0] = sm[lane];
+                s.v[1] = robust ? sm[kBlock + lane] : 0.0;
+                for (int i = lane + 32; i - lane < used; i += 32) {
+                    o.v[0] = sm[i];
+                    o.v[1] = robust ? sm[kBlock + i] : 0.0;
+                    acc_merge_m<kSlotNorm>(s, o, type);
+                }
+#pragma unroll
+                for (int off = 16; off > 0; off >>= 1) acc_shfl_down<kSlotNorm>(s, off, type);
+                if (lane == 0) out[0] = s.v[0], out[1] = s.v[1];
             }
+        }
+    }
+    if constexpr ((SLOTS & kSlotD2) != 0) {
+        if (warp == 1) {
+            const double s = plain(sm + 2 * kBlock);
+            if (lane == 0) out[2] = s;
         }
     }
 }
 
-template <bool S>
-__global__ void __launch_bounds__(kBlock, MTJG_PERSIST_MINB) k_cg_persist(PersistCg c, int normtype)
+// This CTA's partials of a phase: out[k] is slot k's (rows_reduce).  By the
+// warps that summed them.
+template <int SLOTS, int SL>
+__device__ __forceinline__ void publish(const PersistCg &c, int phase, int t0, int G, const double (*out)[4], int type)
+{
+    const int tid = threadIdx.x;
+#pragma unroll
+    for (int k = 0; k < SL; ++k) {
+        if (t0 + k * G >= c.pt.num_tiles) continue;
+        const int t = t0 + k * G;
+        const unsigned long long tag = (unsigned long long)phase + 1;
+        if ((SLOTS & kSlotNorm) != 0 && tid == 0) {
+            st_packet(partial(c, phase, 0, t), out[k][0], tag);
+            if (type == MTJG_NORM_TWO_ROBUST) st_packet(partial(c, phase, 1, t), out[k][1], tag);
+        }
+        if ((SLOTS & kSlotD2) != 0 && tid == 32) st_packet(partial(c, phase, 2, t), out[k][2], tag);
+    }
+}
+
+// system_sum over the tiles' partials of a phase, waiting for each with all
+// of a thread's loads in flight; in out[0..2] after the barrier it ends with.
+template <int SLOTS>
+__device__ void collect(const PersistCg &c, int phase, int type, double *sm, double *out, int *s_bad)
+{
+    constexpr bool kN = (SLOTS & kSlotNorm) != 0;
+    constexpr int kMost = (kPersistMaxTiles + kBlock - 1) / kBlock;
+    const int NT = c.pt.num_tiles;
+    const bool robust = type == MTJG_NORM_TWO_ROBUST;
+    const unsigned long long tag = (unsigned long long)phase + 1;
+    Acc s;
+    acc_zero(s);
+    if ((int)threadIdx.x < NT) {
+        // every packet of the thread is read again until all are there: one
+        // round trip a round, however many are late
+        Acc o[kMost];
+        for (long long i = 0;; ++i) {
+            bool late = false;
+#pragma unroll
+            for (int u = 0; u < kMost; ++u) {
+                const int i1 = (int)threadIdx.x + u * kBlock, t = i1 < NT ? i1 : (int)threadIdx.x;
+                acc_zero(o[u]);
+                if (kN) {
+                    const ulonglong2 n = ld_packet(partial(c, phase, 0, t));
+                    late |= n.y != tag;
+                    o[u].v[0] = __longlong_as_double((long long)n.x);
+                    if (robust) {
+                        const ulonglong2 q = ld_packet(partial(c, phase, 1, t));
+                        late |= q.y != tag;
+                        o[u].v[1] = __longlong_as_double((long long)q.x);
+                    }
+                }
+                const ulonglong2 d = ld_packet(partial(c, phase, 2, t));
+                late |= d.y != tag;
+                o[u].v[2] = __longlong_as_double((long long)d.x);
+            }
+            if (!late || !wait_on(c, i, s_bad)) break;
+        }
+#pragma unroll
+        for (int u = 0; u < kMost; ++u)
+            if ((int)threadIdx.x + u * kBlock < NT) acc_merge_m<SLOTS>(s, o[u], type);
+    }
+    rows_reduce<SLOTS>(s, NT < kBlock ? NT : kBlock, type, sm, out);
+    rows_sync();
+}
+
+// SL product tiles per CTA (tile bid + k G in slot k).  The last warp runs
+// the monitor's test (a square root, divisions and compares on the narrow
+// FP64 pipe, 2400 cycles) beside the next product, whose p and q a solve that
+// has ended leaves unused.
+constexpr int kPersistBlock = kBlock + 32;
+
+template <bool S, int SL>
+__global__ void __launch_bounds__(kPersistBlock, MTJG_PERSIST_MINB) k_cg_persist(PersistCg c, int normtype)
 {
     extern __shared__ __align__(16) unsigned char slots[];
-    __shared__ double red_sm[kParts * kBlock];
+    // (the collecting sums have a place of their own: the threads that poll
+    // nothing reach theirs while warps 0 and 1 still sum the CTA's partial)
+    __shared__ double red_sm[3 * kBlock], all_sm[3 * kBlock];
+    __shared__ double s_q[SL][kBlock];
+    __shared__ double s_out[SL][4], s_sum[4], s_beta, s_alpha;
     __shared__ SysState s_st;
-    __shared__ int s_run;  // the running count of CTAs other than 0 (unused)
-    const int tid = threadIdx.x, G = (int)gridDim.x, bid = (int)blockIdx.x;
+    __shared__ int s_run, s_bad;  // s_run: the running count of CTAs other than 0 (unused)
+    const int tid = threadIdx.x, G = (int)gridDim.x, bid = (int)blockIdx.x, NT = c.pt.num_tiles;
+    const bool rows_thread = tid < kBlock;
+    const int nt = normtype;
     if (tid == 0) {
         s_st = c.m.st[0];
         s_run = 1;
+        s_bad = 0;
     }
     // this CTA's product tiles into their slots (entries and rows checked
-    // against the slot: a tile that does not fit stops the solve)
-    int bad = 0;
-    for (int k = 0; k < c.slots; ++k) {
+    // against the slot: a tile that does not fit stops the solve), its rows'
+    // vectors into registers: row r0 + tid of each tile
+    int bad = 0, row[SL], r0s[SL], rows[SL];
+    double xv[SL], rv[SL], zv[SL], iv[SL], pv[SL];
+    const bool jac = c.pc == kPcJacobi;
+#pragma unroll
+    for (int k = 0; k < SL; ++k) {
         const int t = bid + k * G;
-        if (t >= c.pt.num_tiles) break;
+        row[k] = -1;
+        rows[k] = r0s[k] = 0;
+        xv[k] = rv[k] = zv[k] = iv[k] = pv[k] = 0.0;
+        if (t >= NT) continue;
         unsigned char *slot = slots + (size_t)k * kSlotBytes;
         const int r0 = c.pt.tile_row[t], r1 = c.pt.tile_row_end[t];
         const int nz0 = __ldg(c.A.rowptr + r0), nz1 = __ldg(c.A.rowptr + r1);
@@ -244,11 +340,24 @@ __global__ void __launch_bounds__(kBlock, MTJG_PERSIST_MINB) k_cg_persist(Persis
         double *sv = reinterpret_cast<double *>(slot);
         int *sc = reinterpret_cast<int *>(slot + kSlotValBytes);
         int *sr = reinterpret_cast<int *>(slot + kSlotValBytes + kSlotColBytes);
-        for (int i = tid; i <= r1 - r0; i += kBlock) sr[i] = __ldg(c.A.rowptr + r0 + i) - nz0;
-        for (int e = tid; e < nz1 - nz0; e += kBlock) {
+        for (int i = tid; i <= r1 - r0; i += kPersistBlock) sr[i] = __ldg(c.A.rowptr + r0 + i) - nz0;
+        for (int e = tid; e < nz1 - nz0; e += kPersistBlock) {
             sv[e] = __ldg(c.A.val + nz0 + e);
             sc[e] = __ldg(c.A.colind + nz0 + e);
         }
+        r0s[k] = r0;
+        rows[k] = r1 - r0;
+        if (rows_thread && tid < r1 - r0) {
+            const int r = r0 + tid;
+            row[k] = r;
+            xv[k] = c.x[r];
+            rv[k] = c.r[r];
+            zv[k] = jac ? c.z[r] : rv[k];
+            iv[k] = jac ? __ldg(c.invdiag + r) : 0.0;
+        }
+        // tags of an earlier launch go
+        if (tid < 3) st_packet(partial(c, 0, tid, t), 0.0, 0ull), st_packet(partial(c, 1, tid, t), 0.0, 0ull);
+        if (rows_thread && tid < r1 - r0) st_packet(c.p + r0 + tid, 0.0, 0ull);
     }
     if (__syncthreads_or(bad)) {
         if (tid == 0) {
@@ -257,67 +366,144 @@ __global__ void __launch_bounds__(kBlock, MTJG_PERSIST_MINB) k_cg_persist(Persis
         }
         return;
     }
-    CgQ<S> qop{nullptr, c.q, &s_st};
+    // every tag is cleared before any packet is published
+    if (!grid_barrier(c.gb, (unsigned long long)G, c.err)) return;
     MonPtrs m = c.m;
     m.st = &s_st;
     if (bid != 0) {
         m.mon.hist_cap = 0;
         m.num_running = &s_run;
     }
-    CgUpd<S> uop{c.x, c.r, c.z, nullptr, c.q, c.invdiag, c.pc, m};
-    const int nt = normtype;
-    unsigned long long target = 0;
-    int par = 0;  // p[par] holds the previous iteration's p
-    while (s_st.status == ST_RUNNING) {
-        const double *po = c.p[par];
-        double *pn = c.p[par ^ 1];
-        // p = z (first) or beta p + z, formed in the gathers; q = A p and the
-        // p.q partials, one tile (group) at a time
-        {
-            const bool first = s_st.iter == 0;
-            const double beta = s_st.beta;
-            for (int k = 0; k < c.slots; ++k) {
+    constexpr int kSlotsQ = OpSlots<CgQ<S>>::value, kSlotsU = OpSlots<CgUpd<S>>::value;
+    constexpr int kBatch = 8;  // entries whose packets are in flight at once
+    int phase = 0;
+    unsigned long long it = 1;  // the coming p's tag
+    bool first = true;
+    double rho = s_st.rho;  // thread 0's
+    if (s_st.status != ST_RUNNING) return;
+    for (;;) {
+        if (rows_thread) {
+            if (tid == 0 && !first) {  // beta = rho / rho_1, rho = r.z
+                const double rz = s_sum[2];
+                s_beta = rz / rho;
+                rho = rz;
+            }
+            rows_sync();
+            const double beta = s_beta;
+            // p = z (first) or beta p + z, out to the tiles that gather it
+#pragma unroll
+            for (int k = 0; k < SL; ++k) {
+                pv[k] = first ? zv[k] : fmac<S>(pv[k], beta, zv[k]);
+                if (row[k] >= 0) {
+                    st_packet(c.p + row[k], pv[k], it);
+                    s_q[k][tid] = pv[k];
+                }
+            }
+            // q = A p and the p.q partials
+#pragma unroll
+            for (int k = 0; k < SL; ++k) {
                 const int t = bid + k * G;
-                if (t >= c.pt.num_tiles) break;
-                const unsigned char *slot = slots + (size_t)k * kSlotBytes;
-                Acc acc;
-                acc_zero(acc);
-                const int vec = S ? 1 : (c.pt.group_info[t] & 0xff);
-                if (vec == 1)
-                    pcg_tile<S, 1>(c, qop, slot, t, po, pn, first, beta, acc);
-                else if (vec == 4)
-                    pcg_tile<S, 4>(c, qop, slot, t, po, pn, first, beta, acc);
-                else
-                    pcg_tile<S, 32>(c, qop, slot, t, po, pn, first, beta, acc);
-                group_partial<OpSlots<CgQ<S>>::value>(acc, t, c.rcq, nt, red_sm);
+                Acc part;
+                acc_zero(part);
+                bool one = true;
+                if (t < NT) {
+                    const unsigned char *slot = slots + (size_t)k * kSlotBytes;
+                    const double *sv = reinterpret_cast<const double *>(slot);
+                    const int *sc = reinterpret_cast<const int *>(slot + kSlotValBytes);
+                    const int *sr = reinterpret_cast<const int *>(slot + kSlotValBytes + kSlotColBytes);
+                    const int vec = S ? 1 : (c.pt.group_info[t] & 0xff);
+                    one = vec == 1;
+                    double sum = 0.0;
+                    if (one) {
+                        if (row[k] >= 0) {
+                            const int b = sr[tid], e = sr[tid + 1];
+                            for (int i0 = b; i0 < e; i0 += kBatch) {
+                                ulonglong2 g[kBatch];
+#pragma unroll
+                                for (int u = 0; u < kBatch; ++u) g[u] = ld_packet(c.p + sc[i0 + u < e ? i0 + u : i0]);
+#pragma unroll
+                                for (int u = 0; u < kBatch; ++u)
+                                    if (i0 + u < e)
+                                        sum = fmac<S>(sv[i0 + u],
+                                                      g[u].y == it ? __longlong_as_double((long long)g[u].x)
+                                                                   : wait_packet(c, c.p + sc[i0 + u], it, &s_bad),
+                                                      sum);
+                            }
+                            const double q = mtj_assign(sum);
+                            s_q[k][tid] = q;
+                            part.v[2] = fmac<S>(pv[k], q, part.v[2]);
+                        }
+                    } else {
+                        // 4 or 32 lanes per row, strided entries and k_spmv's butterfly
+                        const int gg = vec == 4 ? tid >> 2 : tid >> 5, l = vec == 4 ? tid & 3 : tid & 31;
+                        const bool in = gg < rows[k];
+                        rows_sync();  // the rows' p is in s_q
+                        if (in)
+                            for (int i = sr[gg] + l; i < sr[gg + 1]; i += vec)
+                                sum = fmac<S>(sv[i], wait_packet(c, c.p + sc[i], it, &s_bad), sum);
+                        for (int off = vec / 2; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off, vec);
+                        if (in && l == 0) {
+                            const double q = mtj_assign(sum);
+                            part.v[2] = fmac<S>(s_q[k][gg], q, part.v[2]);
+                            s_q[k][gg] = q;
+                        }
+                    }
+                }
+                // (rows of several lanes each are spread over the whole block)
+                rows_reduce<kSlotsQ>(part, one ? rows[k] : kBlock, nt, red_sm, s_out[k]);
+                if (SL > 1) rows_sync();
             }
+        } else if (!first && tid == kBlock) {  // the last update's test
+            s_st.rho_1 = s_st.rho;
+            s_st.iter++;
+            const int code = m.check(s_st, 0, norm_finish(s_sum, nt));
+            if (code == ST_RUNNING) s_st.rho = s_sum[2];
+            m.finish(s_st, code);
         }
-        target += (unsigned long long)G;
-        if (!grid_barrier(c.gb, target, c.err)) break;
-        {
-            const Acc s = system_sum<OpSlots<CgQ<S>>::value>(c.rcq, 0, nt, red_sm);
-            if (tid == 0) qop.scalar(0, s);
-            __syncthreads();
-        }
-        // x += alpha p, r -= alpha q, z = M r with the |r| and r.z partials
-        {
-            const double al = s_st.alpha;
-            for (int t = bid; t < c.rt.num_tiles; t += G) {
-                Acc acc;
-                acc_zero(acc);
-                pcg_update<S>(c, pn, t, al, nt, acc);
-                group_partial<OpSlots<CgUpd<S>>::value>(acc, t, c.rcu, nt, red_sm);
+        __syncthreads();
+        if (s_st.status != ST_RUNNING) break;
+        if (rows_thread) {
+            publish<kSlotsQ, SL>(c, phase, bid, G, s_out, nt);
+            collect<kSlotsQ>(c, phase, nt, all_sm, s_sum, &s_bad);
+            ++phase;
+            if (tid == 0) s_alpha = rho / s_sum[2];
+            rows_sync();
+            // x += alpha p, r -= alpha q, z = M r with the |r| and r.z partials
+            const double al = s_alpha;
+#pragma unroll
+            for (int k = 0; k < SL; ++k) {
+                Acc part;
+                acc_zero(part);
+                if (row[k] >= 0) {
+                    double rr = rv[k];
+                    if (al != 0) {
+                        xv[k] = fmac<S>(al, pv[k], xv[k]);
+                        rr = fmac<S>(-al, s_q[k][tid], rr);
+                        rv[k] = rr;
+                    }
+                    norm_add<S>(part, rr, nt);
+                    zv[k] = rr;
+                    if (jac) zv[k] = rr * iv[k];
+                    part.v[2] = fmac<S>(rr, zv[k], part.v[2]);
+                }
+                rows_reduce<kSlotsU>(part, rows[k], nt, red_sm, s_out[k]);
+                if (SL > 1) rows_sync();
             }
+            publish<kSlotsU, SL>(c, phase, bid, G, s_out, nt);
+            collect<kSlotsU>(c, phase, nt, all_sm, s_sum, &s_bad);
+            ++phase;
         }
-        target += (unsigned long long)G;
-        if (!grid_barrier(c.gb, target, c.err)) break;
-        {
-            const Acc s = system_sum<OpSlots<CgUpd<S>>::value>(c.rcu, 0, nt, red_sm);
-            if (tid == 0) uop.scalar(0, s);
-            __syncthreads();
-        }
-        par ^= 1;
+        __syncthreads();
+        if (s_bad) return;
+        first = false;
+        ++it;
     }
+#pragma unroll
+    for (int k = 0; k < SL; ++k)
+        if (row[k] >= 0) {
+            c.x[row[k]] = xv[k];
+            c.r[row[k]] = rv[k];
+        }
     if (bid == 0 && tid == 0) c.m.st[0] = s_st;
 }
 

@@ -703,12 +703,11 @@ struct mtjg_solver {
     int64_t ir_fcap = 0, ir_dcap = 0, ir_hcap = 0;
     bool last_empty = false;   // the last solve had n == 0: its history is empty_it (residuals 0)
     std::vector<int> empty_it;
-    // one-launch CG (persist.cuh): MTJG_LAUNCH_*, the product's partials,
-    // the barrier's arrival count and abort word
+    // one-launch CG (persist.cuh): MTJG_LAUNCH_*, its packets, the barrier's
+    // arrival count and abort word
     int launch_mode = MTJG_LAUNCH_AUTO;
-    double *pc_part = nullptr;
-    int64_t pc_part_cap = 0;
-    double *pc_p2 = nullptr;  // the second p buffer
+    ulonglong2 *pc_packets = nullptr;
+    int64_t pc_cap = 0;
     unsigned long long *pc_bar = nullptr;
     bool last_persistent = false;
     unsigned long long *gm_bar = nullptr;  // the one-launch Gram-Schmidt's barrier (gmres.cuh)
@@ -747,6 +746,15 @@ int pc_mode(const mtjg_solver *S)
     if (!S->M || S->M->kind == MTJG_PC_IDENTITY) return kPcIdentity;
     if (S->M->kind == MTJG_PC_JACOBI) return kPcJacobi;
     return kPcExternal;
+}
+
+// One system of at most kPersistMaxTiles product tiles, no row longer than a
+// tile, each tile a reduction group: CG's row phases take its product tiles,
+// as the one-launch CG does.
+bool small_cg(const mtjg_csr *A)
+{
+    return A->sys_rows.empty() && A->tiles.num_sys == 1 && A->tiles.num_long == 0 && A->tiles.num_tiles > 0 &&
+           A->tiles.num_tiles <= kPersistMaxTiles && A->tiles.num_groups == A->tiles.num_tiles;
 }
 
 template <bool STRICT>
@@ -796,14 +804,15 @@ struct Phases {
     {
         const int pcm = pc_mode(S);
         double *z = pcm == kPcIdentity ? v(V_R) : v(V_Z);
+        const TileSet &rt = pcm != kPcExternal && small_cg(A) ? A->tiles : A->rtiles;
         if (pcm == kPcExternal) {
             int st = pc(v(V_R), z, &S->st->status);
             if (st != MTJG_OK) return st;
             PH_CHECK(launch_rows(S->ctx, A->rtiles, CgDot<STRICT>{v(V_R), z, S->st}, rc(), norm()));
         }
-        PH_CHECK(launch_rows(S->ctx, A->rtiles, CgP<STRICT>{v(V_P), z, S->st}, rc(), norm()));
+        PH_CHECK(launch_rows(S->ctx, rt, CgP<STRICT>{v(V_P), z, S->st}, rc(), norm()));
         PH_CHECK(launch_spmv(S->ctx, csr(), A->tiles, v(V_P), CgQ<STRICT>{v(V_P), v(V_Q), S->st}, rc(), norm()));
-        PH_CHECK(launch_rows(S->ctx, A->rtiles,
+        PH_CHECK(launch_rows(S->ctx, rt,
                              CgUpd<STRICT>{v(V_X), v(V_R), z, v(V_P), v(V_Q), invdiag(), pcm, mp()}, rc(), norm()));
         return MTJG_OK;
     }
@@ -1258,16 +1267,13 @@ int ensure_state(mtjg_solver *S, int ns)
     return MTJG_OK;
 }
 
-// CG with the identity or Jacobi preconditioner on one system of at most
-// kPersistMaxTiles product tiles (no row longer than a tile) runs its loop in
-// one cooperative launch (persist.cuh) unless the graph path was asked for.
+// CG with the identity or Jacobi preconditioner on a small system runs its
+// loop in one cooperative launch (persist.cuh) unless the graph path was
+// asked for.
 bool persistent_cg(const mtjg_solver *S, const mtjg_csr *A)
 {
     return S->launch_mode == MTJG_LAUNCH_AUTO && S->kind == MTJG_CG && !S->mixed && !S->xmon &&
-           pc_mode(S) != kPcExternal &&
-           A->sys_rows.empty() && A->tiles.num_sys == 1 && A->rtiles.num_sys == 1 && A->tiles.num_long == 0 &&
-           A->tiles.num_tiles > 0 && A->tiles.num_tiles <= kPersistMaxTiles &&
-           A->tiles.num_groups == A->tiles.num_tiles && A->rtiles.num_groups == A->rtiles.num_tiles;
+           pc_mode(S) != kPcExternal && small_cg(A);
 }
 
 struct PersistPlan {
@@ -1276,34 +1282,25 @@ struct PersistPlan {
     size_t smem = 0;
 };
 
-// The grid of the one-launch CG: as many co-resident CTAs as there are
-// tiles, up to 4 per SM, each caching ceil(tiles / grid) product tiles in
-// shared memory; fewer CTAs per SM (more slots each) when that does not fit.
-// False when no grid fits: the solve takes the graph path.
+// The grid of the one-launch CG: a CTA per product tile where they are all
+// co-resident, else two tiles each.  False when no grid fits: the solve takes
+// the graph path.
 template <bool STRICT>
 bool persist_plan(mtjg_ctx *ctx, const mtjg_csr *A, PersistPlan &pl)
 {
-    auto k = k_cg_persist<STRICT>;
-    int optin = 0;
-    cudaFuncAttributes fa{};
-    if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device) != cudaSuccess ||
-        cudaFuncGetAttributes(&fa, k) != cudaSuccess)
-        return false;
-    const int maxdyn = optin - (int)fa.sharedSizeBytes;
-    if (maxdyn < kSlotBytes || cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, maxdyn) != cudaSuccess)
-        return false;
-    const int NT = A->tiles.num_tiles, NR = A->rtiles.num_tiles;
-    for (int per_sm = 4; per_sm >= 1; --per_sm) {
-        const int G = std::min(std::max(NT, NR), per_sm * ctx->num_sms);
-        const int slots = (NT + G - 1) / G;
-        const size_t smem = (size_t)slots * kSlotBytes;
-        if (smem > (size_t)maxdyn) continue;
+    for (int slots = 1; slots <= 2; ++slots) {
+        auto k = slots == 1 ? k_cg_persist<STRICT, 1> : k_cg_persist<STRICT, 2>;
+        const int smem = slots * kSlotBytes, G = (A->tiles.num_tiles + slots - 1) / slots;
         int blocks = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k, kBlock, smem) != cudaSuccess) return false;
+        if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k, kPersistBlock, smem) != cudaSuccess) {
+            (void)cudaGetLastError();
+            return false;
+        }
         if ((int64_t)blocks * ctx->num_sms >= G) {
             pl.grid = G;
             pl.slots = slots;
-            pl.smem = smem;
+            pl.smem = (size_t)smem;
             return true;
         }
     }
@@ -1321,40 +1318,36 @@ template <bool STRICT>
 int run_persistent_cg(mtjg_solver *S, mtjg_csr *A, const PersistPlan &pl)
 {
     mtjg_ctx *ctx = S->ctx;
-    const int64_t need = (int64_t)(A->tiles.num_groups + 1) * kParts;
-    if (need > S->pc_part_cap) {
-        cudaFree(S->pc_part);
-        S->pc_part = nullptr;
-        S->pc_part_cap = 0;
-        MTJG_CUDA(cudaMalloc(&S->pc_part, sizeof(double) * (size_t)need));
-        S->pc_part_cap = need;
+    // packets of 16 bytes: p of each row, the partials' two sets
+    const int64_t need = (int64_t)S->n + 2 * kPacketStride * (int64_t)A->tiles.num_tiles;
+    if (need > S->pc_cap) {
+        cudaFree(S->pc_packets);
+        S->pc_packets = nullptr;
+        S->pc_cap = 0;
+        MTJG_CUDA(cudaMalloc(&S->pc_packets, sizeof(ulonglong2) * (size_t)need));
+        S->pc_cap = need;
     }
-    if (!S->pc_p2) MTJG_CUDA(cudaMalloc(&S->pc_p2, sizeof(double) * (size_t)std::max(1, S->n)));
     if (!S->pc_bar) MTJG_CUDA(cudaMalloc(&S->pc_bar, 2 * sizeof(unsigned long long)));
     MTJG_CUDA(cudaMemsetAsync(S->pc_bar, 0, 2 * sizeof(unsigned long long), ctx->stream));
     const int pcm = pc_mode(S);
     PersistCg c;
     c.A = CsrArgs{A->rowptr, A->colind, A->val};
     c.pt = tile_args(A->tiles);
-    c.rt = tile_args(A->rtiles);
     c.invdiag = S->M && S->M->kind == MTJG_PC_JACOBI ? S->M->invdiag : nullptr;
     c.x = S->vecs[V_X];
     c.r = S->vecs[V_R];
     c.z = pcm == kPcIdentity ? S->vecs[V_R] : S->vecs[V_Z];
-    c.q = S->vecs[V_Q];
-    c.p[0] = S->vecs[V_P];
-    c.p[1] = S->pc_p2;
     c.pc = pcm;
-    c.slots = pl.slots;
-    c.rcq = RedCtx{S->pc_part, A->cnt, A->tiles.sys_group, A->num_running};
-    c.rcu = red_ctx(A, A->rtiles);
+    c.p = S->pc_packets;
+    c.part = S->pc_packets + S->n;
     c.m = MonPtrs{S->st, mon_dev(S), S->hist_r, S->hist_it, A->num_running};
     c.gb = GridBar{S->pc_bar, reinterpret_cast<int *>(S->pc_bar + 1)};
     c.err = ctx->d_flag;
     int normtype = S->mon.norm;
     void *args[] = {&c, &normtype};
-    const cudaError_t e = cudaLaunchCooperativeKernel(reinterpret_cast<void *>(k_cg_persist<STRICT>), dim3(pl.grid),
-                                                      dim3(kBlock), args, pl.smem, ctx->stream);
+    void *k = pl.slots == 1 ? reinterpret_cast<void *>(k_cg_persist<STRICT, 1>)
+                            : reinterpret_cast<void *>(k_cg_persist<STRICT, 2>);
+    const cudaError_t e = cudaLaunchCooperativeKernel(k, dim3(pl.grid), dim3(kPersistBlock), args, pl.smem, ctx->stream);
     if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported) {
         (void)cudaGetLastError();  // a launch-configuration error: nothing ran, nothing is sticky
         return kCoopRefused;
@@ -1807,8 +1800,7 @@ extern "C" int mtjg_solver_destroy(mtjg_solver *S)
     drop_graph(S);
     for (double *p : S->vecs) cudaFree(p);
     for (float *p : S->v32) cudaFree(p);
-    cudaFree(S->pc_part);
-    cudaFree(S->pc_p2);
+    cudaFree(S->pc_packets);
     cudaFree(S->pc_bar);
     cudaFree(S->invdiag32);
     cudaFree(S->V);
