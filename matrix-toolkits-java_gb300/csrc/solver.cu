@@ -251,6 +251,7 @@ struct BiInit {  // r = b - A x; rtilde = r (:71-72); first test; rho_1 = rtilde
     MonPtrs m;
     static constexpr bool kReduce = true;
     static constexpr bool kNeedsXr = false;
+    static constexpr int kSlots = kSlotNorm | kSlotD2;
     __device__ bool active(int) const { return true; }
     __device__ double init(int, int) const { return 0.0; }
     __device__ void row(int i, int, double d, double, Acc &a) const
@@ -306,6 +307,7 @@ struct BiV {  // v = A phat; alpha = rho_1 / rtilde.v (:98-99)
     SysState *st;
     static constexpr bool kReduce = true;
     static constexpr bool kNeedsXr = false;
+    static constexpr int kSlots = kSlotD2;
     __device__ bool active(int sys) const { return st[sys].status == ST_RUNNING; }
     __device__ double init(int, int) const { return 0.0; }
     __device__ void row(int i, int, double d, double, Acc &a) const
@@ -329,6 +331,7 @@ struct BiS {  // s = r - alpha v; x += alpha phat; test on s (:100-104); fused s
     MonPtrs m;
     static constexpr bool kReduce = true;
     static constexpr bool kNeedsXr = false;
+    static constexpr int kSlots = kSlotNorm;
     __device__ bool active(int sys) const { return m.st[sys].status == ST_RUNNING; }
     __device__ void row(int i, int sys, Acc &a) const
     {
@@ -356,6 +359,7 @@ struct BiT {  // t = A shat; omega = t.s / t.t (:107-108)
     SysState *st;
     static constexpr bool kReduce = true;
     static constexpr bool kNeedsXr = false;
+    static constexpr int kSlots = kSlotD2 | kSlotD3;
     __device__ bool active(int sys) const { return st[sys].status == ST_RUNNING; }
     __device__ double init(int, int) const { return 0.0; }
     __device__ void row(int i, int, double d, double, Acc &a) const
@@ -379,6 +383,7 @@ struct BiR {  // x += omega shat; r = s - omega t (:109-110); next test; rho_1, 
     MonPtrs m;
     static constexpr bool kReduce = true;
     static constexpr bool kNeedsXr = false;
+    static constexpr int kSlots = kSlotNorm | kSlotD2;
     __device__ bool active(int sys) const { return m.st[sys].status == ST_RUNNING; }
     __device__ void row(int i, int sys, Acc &a) const
     {
@@ -480,6 +485,7 @@ struct GmNorm {
     bool first;
     static constexpr bool kReduce = true;
     static constexpr bool kNeedsXr = false;
+    static constexpr int kSlots = kSlotNorm | kSlotD2;
     __device__ bool active(int sys) const { return first || m.st[sys].status == ST_RUNNING; }
     __device__ void row(int i, int, Acc &a) const
     {
@@ -545,6 +551,7 @@ struct GmMgs {
     GmData g;
     static constexpr bool kReduce = true;
     static constexpr bool kNeedsXr = false;
+    static constexpr int kSlots = kSlotD2;
     __device__ bool active(int sys) const { return m.st[sys].gate == ST_RUNNING; }
     __device__ void row(int r, int, Acc &a) const
     {
