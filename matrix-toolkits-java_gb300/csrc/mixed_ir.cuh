@@ -96,7 +96,7 @@ struct IrInner {
             int st = pc(p, ph, &php);
             if (st != MTJG_OK) return st;
             if ((st = prod(php, v, nullptr)) != MTJG_OK) return st;
-            k_ir_vdot<<<dim3(G, 1), kIrBlock, 0, stream()>>>(n, rin, 0, v, part);
+            k_ir_vdot<<<dim3(G, 1), kIrBlock, 0, stream()>>>(n, rin, 0, 1, v, part);
             count();
             finish(1);
             if ((st = wait()) != MTJG_OK) return st;
@@ -153,7 +153,7 @@ struct IrInner {
                 // classical Gram-Schmidt, twice; the coefficients of both passes
                 // land in dev[0..j] and dev[j+1..2j+1], ||w||^2 in dev[2j+2]
                 for (int pass = 0; pass < 2; ++pass) {
-                    k_ir_vdot<<<dim3(G, j + 1), kIrBlock, 0, stream()>>>(n, V, ld, ww, part);
+                    k_ir_vdot<<<dim3(G, (j + kIrDots) / kIrDots), kIrBlock, 0, stream()>>>(n, V, ld, j + 1, ww, part);
                     count();
                     k_ir_final<<<j + 1, 32, 0, stream()>>>(part, G, dev + pass * (j + 1));
                     count();

@@ -20,16 +20,47 @@ __device__ __forceinline__ double ir_block_sum(double v, double *sm)
     return s;
 }
 
-// part[y * gridDim.x + block] = block's share of V_y . w  (grid: G x k)
-__global__ void __launch_bounds__(kIrBlock) k_ir_vdot(int n, const float *V, int64_t ldv, const float *w, double *part)
+// (double)f by integer operations where f is normal or zero: a conversion
+// takes the narrow FP64 pipe as long as a multiply-add does.
+__device__ __forceinline__ double ir_widen(float f)
+{
+    const unsigned u = __float_as_uint(f), m = u & 0x7fffffffu;
+    if (m - 0x00800000u >= 0x7f000000u && m != 0u) return (double)f;  // subnormal, infinity or NaN
+    const unsigned hi = (u & 0x80000000u) | ((m >> 3) + (m != 0u ? 0x38000000u : 0u));
+    return __hiloint2double((int)hi, (int)(u << 29));
+}
+
+// part[y * gridDim.x + block] = block's share of V_y . w for kIrDots vectors
+// a block (grid: G x k / kIrDots, rounded up): w is read and widened once for
+// all of them.  250,047 rows, 1 to 31 vectors: 29 us a launch on average with
+// a block per vector and two conversions a product (three FP64 operations,
+// 19 us of that pipe), 22 us so.
+constexpr int kIrDots = 4;
+__global__ void __launch_bounds__(kIrBlock) k_ir_vdot(int n, const float *V, int64_t ldv, int k, const float *w,
+                                                      double *part)
 {
     __shared__ double sm[kIrBlock / 32];
-    const float *v = V + (int64_t)blockIdx.y * ldv;
-    double acc = 0.0;
-    for (int i = blockIdx.x * kIrBlock + threadIdx.x; i < n; i += gridDim.x * kIrBlock)
-        acc += (double)v[i] * (double)w[i];
-    acc = ir_block_sum(acc, sm);
-    if (threadIdx.x == 0) part[(size_t)blockIdx.y * gridDim.x + blockIdx.x] = acc;
+    const int y0 = (int)blockIdx.y * kIrDots, left = k - y0;
+    const float *v = V + (int64_t)y0 * ldv;
+    double acc[kIrDots];
+#pragma unroll
+    for (int y = 0; y < kIrDots; ++y) acc[y] = 0.0;
+    for (int i = blockIdx.x * kIrBlock + threadIdx.x; i < n; i += gridDim.x * kIrBlock) {
+        float vf[kIrDots];
+#pragma unroll
+        for (int y = 0; y < kIrDots; ++y) vf[y] = y < left ? v[(int64_t)y * ldv + i] : 0.0f;
+        const double wd = ir_widen(w[i]);
+#pragma unroll
+        for (int y = 0; y < kIrDots; ++y)
+            if (y < left) acc[y] = fma(ir_widen(vf[y]), wd, acc[y]);
+    }
+#pragma unroll
+    for (int y = 0; y < kIrDots; ++y) {
+        if (y >= left) break;
+        const double s = ir_block_sum(acc[y], sm);
+        if (threadIdx.x == 0) part[(size_t)(y0 + y) * gridDim.x + blockIdx.x] = s;
+        __syncthreads();
+    }
 }
 
 // out[slot] = sum over blocks of part[slot * G + block], in block order
@@ -56,8 +87,10 @@ __global__ void __launch_bounds__(kIrBlock) k_ir_lin(int n, float *out, const fl
         if (b) v = fmaf(cb, b[i], v);
         if (c) v = fmaf(cc, c[i], v);
         out[i] = v;
-        s0 += (double)v * (double)v;
-        if (q) s1 += (double)v * (double)q[i];
+        if (!part) continue;
+        const double vd = ir_widen(v);
+        s0 = fma(vd, vd, s0);
+        if (q) s1 = fma(vd, ir_widen(q[i]), s1);
     }
     if (!part) return;
     s0 = ir_block_sum(s0, sm);
