@@ -33,6 +33,7 @@ static void ctx_free(mtjg_ctx *c)
         if (ev) cudaEventDestroy(ev);
     if (c->d_flag) cudaFree(c->d_flag);
     if (c->h_pinned) cudaFreeHost(c->h_pinned);
+    if (c->h_stage) cudaFreeHost(c->h_stage);
     for (cudaStream_t q : c->side)
         if (q) cudaStreamDestroy(q);
     for (cudaEvent_t e : c->join)
@@ -92,7 +93,8 @@ extern "C" int mtjg_ctx_create(int device, mtjg_ctx **out)
     }
     for (auto &ev : c->events) cudaEventCreate(&ev);
     if (cudaMalloc(&c->d_flag, sizeof(int) * 4) != cudaSuccess ||
-        cudaHostAlloc(&c->h_pinned, sizeof(int) * 64, cudaHostAllocDefault) != cudaSuccess) {
+        cudaHostAlloc(&c->h_pinned, sizeof(int) * 64, cudaHostAllocDefault) != cudaSuccess ||
+        cudaHostAlloc(&c->h_stage, 2 * kStageBytes, cudaHostAllocDefault) != cudaSuccess) {
         mtjg_ctx_destroy(c);
         return fail(MTJG_ERR_OUT_OF_MEMORY, "context allocation failed");
     }

@@ -206,6 +206,11 @@ struct LevelSchedule {
 
 }  // namespace mtjg
 
+namespace mtjg {
+constexpr size_t kStageBytes = 128 << 10;
+constexpr int kPinFlag = 63;  // the word of h_pinned for a product's copy of the error flag
+}  // namespace mtjg
+
 // --------------------------------------------------------------- handles
 struct mtjg_ctx {
     std::atomic<int> refs{1};       // the handle itself + every object made with it
@@ -218,6 +223,7 @@ struct mtjg_ctx {
     std::atomic<int64_t> launches{0};  // kernels launched (a serving thread counts here too)
     int *d_flag = nullptr;          // device error flag (bounded waits)
     int *h_pinned = nullptr;        // pinned host words for status polling
+    unsigned char *h_stage = nullptr;  // pinned, 2 kStageBytes: small products on host vectors
     // batched solves run each size of team beside the others (batch.cu);
     // made on first use, ordered on both sides with `stream`
     cudaStream_t side[3] = {};
