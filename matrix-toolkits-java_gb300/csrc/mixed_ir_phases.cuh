@@ -32,15 +32,31 @@ __device__ __forceinline__ double ir_widen(float f)
 
 // part[y * gridDim.x + block] = block's share of V_y . w for kIrDots vectors
 // a block (grid: G x k / kIrDots, rounded up): w is read and widened once for
-// all of them.  250,047 rows, 1 to 31 vectors: 29 us a launch on average with
-// a block per vector and two conversions a product (three FP64 operations,
-// 19 us of that pipe), 22 us so.
+// all of them, and the four butterflies of a warp share their additions (a
+// half, then a quarter of the warp for each vector: 6 FP64 additions and not
+// 20, with the same pairs).  250,047 rows, 1 to 31 vectors: 29.0 us a launch
+// on average with a block per vector and two conversions a product, 21.9 with
+// four vectors and a butterfly each, 14.4 us so.
 constexpr int kIrDots = 4;
+
+// a[y] over the warp, ir_block_sum's pairs: vector 0 in lane 0, 1 in lane 16,
+// 2 in lane 8, 3 in lane 24
+__device__ __forceinline__ double ir_warp_sum4(const double *a, int lane)
+{
+    const bool h = lane & 16, q = lane & 8;
+    const double s01 = (h ? a[1] : a[0]) + __shfl_xor_sync(0xffffffffu, h ? a[0] : a[1], 16);
+    const double s23 = (h ? a[3] : a[2]) + __shfl_xor_sync(0xffffffffu, h ? a[2] : a[3], 16);
+    double s = (q ? s23 : s01) + __shfl_xor_sync(0xffffffffu, q ? s01 : s23, 8);
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    return s;
+}
+
 __global__ void __launch_bounds__(kIrBlock) k_ir_vdot(int n, const float *V, int64_t ldv, int k, const float *w,
                                                       double *part)
 {
-    __shared__ double sm[kIrBlock / 32];
-    const int y0 = (int)blockIdx.y * kIrDots, left = k - y0;
+    __shared__ double sm[kIrDots][kIrBlock / 32];
+    const int y0 = (int)blockIdx.y * kIrDots, left = k - y0, lane = threadIdx.x & 31;
     const float *v = V + (int64_t)y0 * ldv;
     double acc[kIrDots];
 #pragma unroll
@@ -54,12 +70,14 @@ __global__ void __launch_bounds__(kIrBlock) k_ir_vdot(int n, const float *V, int
         for (int y = 0; y < kIrDots; ++y)
             if (y < left) acc[y] = fma(ir_widen(vf[y]), wd, acc[y]);
     }
-#pragma unroll
-    for (int y = 0; y < kIrDots; ++y) {
-        if (y >= left) break;
-        const double s = ir_block_sum(acc[y], sm);
-        if (threadIdx.x == 0) part[(size_t)(y0 + y) * gridDim.x + blockIdx.x] = s;
-        __syncthreads();
+    static_assert(kIrDots == 4, "ir_warp_sum4");
+    const double s = ir_warp_sum4(acc, lane);
+    if ((lane & 7) == 0) sm[(lane >> 4) + 2 * ((lane >> 3) & 1)][threadIdx.x >> 5] = s;
+    __syncthreads();
+    if (threadIdx.x < kIrDots && (int)threadIdx.x < left) {
+        double t = 0.0;
+        for (int q = 0; q < kIrBlock / 32; ++q) t += sm[threadIdx.x][q];
+        part[(size_t)(y0 + threadIdx.x) * gridDim.x + blockIdx.x] = t;
     }
 }
 
