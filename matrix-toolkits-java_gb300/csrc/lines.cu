@@ -522,7 +522,7 @@ __device__ __forceinline__ bool mbar_test_wait(uint64_t *bar, unsigned parity)
 // prepared offsets 104 / 155; operands read inside the chain 96 / 135 (552
 // cycles an L step, of which the four dependent FP64 operations take 300).
 // A whole apply, both permutations included: 633 -> 253 us; 128^3 Poisson
-// ILU 389 -> 355 with the last step; 63^3 FP32 sweeps 248 / 239 -> 39 / 55.
+// ILU 389 -> 355 with the last step; 63^3 FP32 sweeps 248 / 239 -> 33 / 42.
 template <bool S, int MODE, int K, int T, class V>
 __global__ void __launch_bounds__(T + 32 * LinePipe<V>::kLoaders + 32, 1)
     k_line_sweep(const unsigned char *__restrict__ rec, const int *__restrict__ part_step,
@@ -570,15 +570,22 @@ __global__ void __launch_bounds__(T + 32 * LinePipe<V>::kLoaders + 32, 1)
 
     if (tid >= T + 32 * LW) {  // the records and b
         if (lane == 0) {
+            // a few steps at a time: one look at s_done and one fence for all
+            // (a step each: the 63^3 FP32 L sweep 40.5 us, 33.0 so)
+            constexpr int kFew = D / 4;
             int s = 0;
-            for (; s < steps && slot_free(s); ++s) {
-                const size_t ps = (size_t)plan_step(s);
-                uint64_t *bar = &full[s % D];
-                unsigned char *to = slots + (s % D) * kSlot;
+            while (s < steps) {
+                const int end = min(steps, s + kFew);
+                if (!slot_free(end - 1)) break;
                 fence_proxy_async();
-                mbar_arrive_expect_tx(bar, (unsigned)(kRec + kBytesB));
-                bulk_g2s(to, rec + ps * kRec, (unsigned)kRec, bar);
-                bulk_g2s(to + kRec, b + ps * T, (unsigned)kBytesB, bar);
+                for (; s < end; ++s) {
+                    const size_t ps = (size_t)plan_step(s);
+                    uint64_t *bar = &full[s % D];
+                    unsigned char *to = slots + (s % D) * kSlot;
+                    mbar_arrive_expect_tx(bar, (unsigned)(kRec + kBytesB));
+                    bulk_g2s(to, rec + ps * kRec, (unsigned)kRec, bar);
+                    bulk_g2s(to + kRec, b + ps * T, (unsigned)kBytesB, bar);
+                }
             }
             // every copy lands before the block leaves (after an abort the
             // loaders' arrivals may be missing: a bounded wait is enough, the
