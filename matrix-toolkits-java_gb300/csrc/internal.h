@@ -5,6 +5,7 @@
 
 #include <atomic>
 #include <cstdint>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -224,6 +225,7 @@ struct mtjg_ctx {
     int *d_flag = nullptr;          // device error flag (bounded waits)
     int *h_pinned = nullptr;        // pinned host words for status polling
     unsigned char *h_stage = nullptr;  // pinned, 2 kStageBytes: small products on host vectors
+    std::mutex stage_lock;             // held while a product uses h_stage and kPinFlag
     // batched solves run each size of team beside the others (batch.cu);
     // made on first use, ordered on both sides with `stream`
     cudaStream_t side[3] = {};

@@ -826,7 +826,8 @@ static int csr_product_dev(mtjg_csr *A, int op, double alpha, const double *dx, 
 // Vectors of up to kStageBytes go through the context's pinned memory: a
 // pageable copy waits for the stream by itself, and a third wait read the
 // error flag, so a small product was three round trips (2D Poisson 33^2:
-// 36.8 us; 28.8 us with one).
+// 36.8 us; 28.8 us with one).  A thread that finds them in use (products of
+// two matrices of one context at once) copies from and to its own memory.
 static int csr_product_host(mtjg_csr *A, int op, double alpha, const double *x, double *y)
 {
     if (!A || !x || !y) return fail(MTJG_ERR_ILLEGAL_ARGUMENT, "NULL argument");
@@ -834,7 +835,8 @@ static int csr_product_host(mtjg_csr *A, int op, double alpha, const double *x, 
     MTJG_CUDA(cudaSetDevice(ctx->device));
     const bool trans = op >= 2, reads_y = op == 1 || op == 3;
     const size_t bx = sizeof(double) * (size_t)(trans ? A->n : A->m), by = sizeof(double) * (size_t)(trans ? A->m : A->n);
-    const bool stage = bx <= kStageBytes && by <= kStageBytes;
+    std::unique_lock<std::mutex> hold(ctx->stage_lock, std::defer_lock);
+    const bool stage = bx <= kStageBytes && by <= kStageBytes && hold.try_lock();
     unsigned char *sx = ctx->h_stage, *sy = ctx->h_stage + kStageBytes;
     if (stage) {
         std::memcpy(sx, x, bx);
@@ -844,7 +846,7 @@ static int csr_product_host(mtjg_csr *A, int op, double alpha, const double *x, 
     if (reads_y) MTJG_CUDA(cudaMemcpyAsync(A->d_y, stage ? (const void *)sy : y, by, cudaMemcpyHostToDevice, ctx->stream));
     int st = csr_product_dev(A, op, alpha, A->d_x, A->d_y);
     if (st != MTJG_OK) return st;
-    int *flag = ctx->h_pinned + kPinFlag;
+    int own = 0, *flag = stage ? ctx->h_pinned + kPinFlag : &own;
     MTJG_CUDA(cudaMemcpyAsync(stage ? (void *)sy : y, A->d_y, by, cudaMemcpyDeviceToHost, ctx->stream));
     MTJG_CUDA(cudaMemcpyAsync(flag, ctx->d_flag, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
     MTJG_CUDA(cudaStreamSynchronize(ctx->stream));
