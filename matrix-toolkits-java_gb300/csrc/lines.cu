@@ -933,6 +933,11 @@ static int tile_plan(mtjg_ctx *ctx, const TriOp &op, const TriOp &up, TilePlan *
         line_smem<float>(tp->kmax, tp->lanes) + 1024 > optin)
         return done(MTJG_OK, false);
     const int P = tp->parts, T = tp->lanes;
+    // a grid's steps (a part of q by p lines of L rows takes L + q + p - 2):
+    // twice too many, and the lines' offsets (27 ms for 8 x 8 x 2500) are not
+    // worth finding
+    const int64_t likely = (int64_t)P * (n / lines - 2) + (int64_t)(P / ntq) * longest + (int64_t)ntq * planes;
+    if (likely * T > 2 * (2 * (int64_t)n + 65536)) return done(MTJG_OK, false);
     LP_CUDA(cudaMalloc(&pw, sizeof(int) * 2 * (size_t)P));
     LP_CUDA(cudaMalloc(&tp->part_step, sizeof(int) * (size_t)(P + 1)));
     LP_CUDA(cudaMalloc(&tp->pos, sizeof(int) * (size_t)n));
@@ -1037,6 +1042,10 @@ int tile_pair(mtjg_ctx *ctx, const TriOp &lo, const TriOp &up, TilePlan *plan, T
     }
     if (st != MTJG_OK || !t->plan) free_tiles_of(t);
     else *out = t;
+    if (st == MTJG_ERR_OUT_OF_MEMORY) {  // the level schedules take a tenth of the memory
+        (void)cudaGetLastError();
+        st = MTJG_OK;
+    }
     return st;
 }
 
@@ -1115,7 +1124,10 @@ int tile_ilu(mtjg_ctx *ctx, TilePair *t, const TriOp &lo, double *data, bool *fa
     const int64_t count = (int64_t)tp->steps * tp->lanes;
     const size_t bytes = (size_t)tp->steps * mode_record<double, 6>(tp->kmax, tp->lanes);
     unsigned char *rec = nullptr;
-    MTJG_CUDA(cudaMalloc(&rec, bytes + 16));
+    if (cudaMalloc(&rec, bytes + 16) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return MTJG_OK;
+    }
     int *flags = reinterpret_cast<int *>(rec + bytes);  // another column found; zero pivot; the device's error flag
     int h[3] = {1, 1, 1};
     cudaError_t e = cudaMemsetAsync(flags, 0, sizeof(int) * 2, q);

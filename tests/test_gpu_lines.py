@@ -29,7 +29,10 @@ def _banded(n, offsets, rng):
 
 def _ragged(rng):
     """Planes of different line counts, lines of different lengths: an L-shaped grid, natural order."""
-    keep = [(x, y, z) for z in range(7) for y in range(19) for x in range(23) if not (x > 9 + z and y > 11)]
+    return _grid7([(x, y, z) for z in range(7) for y in range(19) for x in range(23) if not (x > 9 + z and y > 11)], rng)
+
+
+def _grid7(keep, rng):
     at = {p: k for k, p in enumerate(keep)}
     rp, ci, v = [0], [], []
     for (x, y, z) in keep:
@@ -65,6 +68,8 @@ def _matrix(name):
     if kind == "nine":  # 2D nine-point: elimination reaches off the diagonal
         N = int(arg)
         return _grid9(N, rng)
+    if kind == "thin":  # 4 x 4 lines: mostly empty lanes, the plan is refused (900: before its offsets are found)
+        return _grid7([(x, y, z) for z in range(int(arg)) for y in range(4) for x in range(4)], rng)
     return getattr(workloads, kind)(int(arg))
 
 
@@ -72,7 +77,7 @@ MATRICES = ["poisson2d:4", "poisson2d:33", "poisson2d:130", "poisson3d:5", "pois
             "convdiff3d:36",  # tiles with empty lanes on two sides
             "banded:-1,0,1", "banded:-50,-1,0,1,50",  # one line, and a value further back than the ring
             "banded:-60,-7,-2,-1,0,1,2,7,60",  # four entries a row, two of them in the line
-            "ragged:", "nine:23"]
+            "ragged:", "nine:23", "thin:100", "thin:200", "thin:900"]
 
 
 def _vectors(n):
@@ -87,7 +92,7 @@ def _vectors(n):
 @pytest.mark.parametrize("name", MATRICES)
 def test_apply(ctx, name, kind):
     n, rp, ci, v = _matrix(name)
-    if kind == "icc" and name.startswith(("banded", "ragged", "nine")):
+    if kind == "icc" and name.startswith(("banded", "ragged", "nine", "thin")):
         v = v.copy()
         rows = np.repeat(np.arange(n), np.diff(rp))
         v[ci != rows] = -1.0  # symmetric
