@@ -1049,7 +1049,7 @@ def run_batch(args):
             "scaling": "weak", "vs_baseline": None, "dtype": "f32+f64", "data": "synthetic",
             "config": {"workload": what, "rows": nt, "nnz": int(A.rowptr[-1]), "seed": seed},
             "fp64": out["fp64"], "mixed": out["mixed"], "mixed_vs_fp64": out["fp64"]["ms"] / out["mixed"]["ms"],
-            "launch": "one persistent launch per solve (each CTA runs whole systems, largest first)",
+            "launch": "persistent launches by system size (teams of CTAs run whole systems, largest first)",
             "tuned_lanes_per_row": dict(sorted(tuned.items()))}
     print(json.dumps(line))
 

@@ -207,8 +207,9 @@ MTJG_API int mtjg_csr_upload_rows(mtjg_ctx *ctx, int num_rows, int num_cols, con
  * `nnz` entries (its class: bands of rows and of entries per row); 0 while
  * no batch of that class has been solved.  A batch from mtjg_batch_upload
  * solved by CG with the identity or Jacobi preconditioner (FP64 or mixed)
- * runs as one persistent launch: each CTA takes whole systems, largest
- * first, and runs their CG to the end.  On the first batch holding a class,
+ * runs as persistent launches: a team of CTAs (one below 4096 rows; 2, 4 or
+ * 8 from 4096, 8192 and 16384) takes whole systems, largest first, and runs
+ * their CG to the end.  On the first batch holding a class,
  * short probe solves time each lanes-per-row candidate; the fastest is kept
  * for the process (MTJG_TUNE=0 in the environment: the entries-per-row rule
  * instead).  No counterpart in the reference. */

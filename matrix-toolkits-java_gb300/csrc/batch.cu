@@ -1,10 +1,10 @@
-// batch.cu -- a batch of independent systems solved by CG in one persistent
-// launch (the batching form): every CTA takes whole systems, largest first,
+// batch.cu -- a batch of independent systems solved by CG in persistent
+// launches (the batching form): teams of CTAs take whole systems, largest first,
 // from a ticket counter and runs each one's complete CG loop on the chip --
 // products, vector updates, fixed-order block reductions, MTJ's monitor --
 // with block barriers only, so thousands of uneven systems need no
 // grid-wide phase, no launch per iteration and no host round trip.  A
-// system's convergence ends its loop (per-system masks), its CTA takes the
+// system's convergence ends its loop (per-system masks), its team takes the
 // next system.
 //
 // Arithmetic per system is that of the CG phases (S/CG.java:58-87 with

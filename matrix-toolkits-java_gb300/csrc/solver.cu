@@ -1490,7 +1490,7 @@ int finish_run(mtjg_solver *S, mtjg_result *res)
 #include "mixed_ir.cuh"
 
 // A batch from mtjg_batch_upload solved by CG with the identity or Jacobi
-// preconditioner runs as one persistent launch (batch.cu); other batches
+// preconditioner runs as persistent launches (batch.cu); other batches
 // run the tiled phases.
 bool batch_persistent(const mtjg_solver *S, const mtjg_csr *A)
 {
