@@ -257,15 +257,9 @@ __global__ void __launch_bounds__(kBlock, EpiCtas<Epi>::value)
                        pb = (unsigned)(p1 - p0) * 4u;
         fence_proxy_async();
         mbar_arrive_expect_tx(&bar[s], vb + cb + pb);
-        // The matrix is read once per product, the vectors by every phase: L2
-        // gives the matrix up first.  128^3 CG + Jacobi 46.6 -> 44.6 ms (its
-        // six vectors are 101 MB, the matrix 183), two products of 150,001
-        // rows and 2.9 M entries 46.8 -> 44.5 us, 48 served requests 58.6 ->
-        // 57.1 ms; mult alone and solves whose matrix stays in L2 unchanged.
-        const uint64_t once = policy_evict_first();
-        if (vb) bulk_g2s(sval(s), d.val + v0, vb, &bar[s], once);
-        if (cb) bulk_g2s(scol(s), d.colind + c0, cb, &bar[s], once);
-        bulk_g2s(srow(s), d.rowptr + p0, pb, &bar[s], once);
+        if (vb) bulk_g2s(sval(s), d.val + v0, vb, &bar[s]);
+        if (cb) bulk_g2s(scol(s), d.colind + c0, cb, &bar[s]);
+        bulk_g2s(srow(s), d.rowptr + p0, pb, &bar[s]);
     };
 
     // The k-th tile of the block's walk lives in stage k % NST.  The first
