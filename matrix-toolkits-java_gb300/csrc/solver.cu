@@ -1569,10 +1569,14 @@ int run_batch(mtjg_solver *S, mtjg_csr *A, mtjg_result *res)
         return cudaMemcpyAsync(S->st, S->last_all.data(), sizeof(SysState) * (size_t)ns, cudaMemcpyHostToDevice,
                                ctx->stream);
     };
-    auto go = [&](const BatchCg &args, std::vector<int> order) -> cudaError_t {
+    // by team size; outlives its copy to the device, which may still read pageable
+    // memory when the call that started it has returned
+    std::vector<int> placed;
+    auto go = [&](const BatchCg &args, const std::vector<int> &order) -> cudaError_t {
         int counts[kTeamSizes];
-        batch_teams(srow, order, counts);
-        cudaError_t e = cudaMemcpyAsync(S->b_order, order.data(), sizeof(int) * order.size(), cudaMemcpyHostToDevice,
+        placed = order;
+        batch_teams(srow, placed, counts);
+        cudaError_t e = cudaMemcpyAsync(S->b_order, placed.data(), sizeof(int) * placed.size(), cudaMemcpyHostToDevice,
                                         ctx->stream);
         if (e == cudaSuccess) e = cudaMemsetAsync(S->b_ticket, 0, sizeof(unsigned) * kTeamSizes, ctx->stream);
         if (e == cudaSuccess) e = batch_launch(ctx, args, counts, S->mixed);
