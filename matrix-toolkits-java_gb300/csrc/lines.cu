@@ -1119,9 +1119,9 @@ int tile_ilu(mtjg_ctx *ctx, TilePair *t, const TriOp &lo, double *data, bool *fa
     const TilePlan *tp = t->plan;
     int optin = 0;
     MTJG_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
-    if (line_smem<double, 6>(tp->kmax, tp->lanes) + 1024 > optin) return MTJG_OK;
-    cudaStream_t q = ctx->stream;
     const int64_t count = (int64_t)tp->steps * tp->lanes;
+    if (line_smem<double, 6>(tp->kmax, tp->lanes) + 1024 > optin || !pivot_pairs_fit(count)) return MTJG_OK;
+    cudaStream_t q = ctx->stream;
     const size_t bytes = (size_t)tp->steps * mode_record<double, 6>(tp->kmax, tp->lanes);
     unsigned char *rec = nullptr;
     if (cudaMalloc(&rec, bytes + 16) != cudaSuccess) {

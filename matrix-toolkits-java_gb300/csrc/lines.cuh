@@ -47,6 +47,13 @@ struct TilePair {
     TileOp op[2];
 };
 
+// Whether the pivots' sweep (tile_ilu) may take a plan of this many positions:
+// its vector holds two values a position, indexed by int.  (The plans' own
+// positions always fit one: with lines of 4 rows and mirrored triangles 2^31
+// entries are at most 859 million rows, and a plan has at most twice the rows
+// and 65536 positions.)
+constexpr bool pivot_pairs_fit(int64_t positions) { return 2 * positions <= 0x7fffffff; }
+
 // Plans the two sweeps; *out stays null when the rows do not form lines (see
 // the rule at tile_plan) and the caller keeps the level schedules.  `plan`:
 // an existing plan of the same factor to use (its transposed sweeps), or null.
