@@ -291,6 +291,7 @@ struct mtjg_precond {
     // FP32 copies for the mixed-precision inner solves (built on first use)
     float *data32 = nullptr, *invdiag32 = nullptr, *y32 = nullptr;
     int64_t v32 = -1;                   // version the copies were made from
+    bool tickets32 = false;             // the FP32 sweeps take lo and up: the tiles' FP32 records did not fit
 };
 
 struct mtjg_solver;

@@ -847,6 +847,16 @@ void free_tiles_of(TilePair *&t)
     t = nullptr;
 }
 
+void tile_drop32(TilePair *t)
+{
+    for (TileOp &op : t->op) {
+        cudaFree(op.rec32);
+        op.rec32 = nullptr;
+    }
+    cudaFree(t->plan->b32);
+    t->plan->b32 = t->plan->y32 = t->plan->x32 = nullptr;
+}
+
 // Tiles of lines pay when rows form lines (kMinLine rows each on average), a
 // record holds every row (kLineK entries), the two triangles mirror each
 // other (so that one plan, walked up and down, serves both sweeps), the tiles

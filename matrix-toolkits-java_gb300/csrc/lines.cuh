@@ -66,6 +66,7 @@ int tile_values(mtjg_ctx *ctx, TilePair *tp, int which, const TriOp &op, const f
 // data as it was.
 int tile_ilu(mtjg_ctx *ctx, TilePair *tp, const TriOp &lo, double *data, bool *factored);
 void free_tiles_of(TilePair *&tp);
+void tile_drop32(TilePair *tp);  // the FP32 records and vectors go
 // x = (second) \ ((first) \ b); x may be b.
 cudaError_t tile_apply(mtjg_ctx *ctx, const TilePair *tp, bool strict, const double *b, double *x, const int *status,
                        int spin);

@@ -739,9 +739,18 @@ int precond_prepare32(mtjg_precond *M)
         MTJG_CUDA(cudaMalloc(&M->y32, sizeof(float) * (size_t)std::max(1, n)));
         if (M->nnz) k_narrow<<<ctx->num_sms * 8, kBlock, 0, ctx->stream>>>(M->nnz, M->data, M->data32);
         ctx->launches++;
+        M->tickets32 = false;
         if (M->tile) {
             int st = tile_values(ctx, M->tile, 0, lower_op(M), M->data32, nullptr);
             if (st == MTJG_OK) st = tile_values(ctx, M->tile, 1, upper_op(M), M->data32, nullptr);
+            if (st == MTJG_ERR_OUT_OF_MEMORY) {
+                // the tickets need a tenth of the records' memory (build_levels frees what it replaces)
+                (void)cudaGetLastError();
+                tile_drop32(M->tile);
+                st = build_levels(ctx, n, 0, 1, M->rowptr, M->colind, M->diag, nullptr, M->lo);
+                if (st == MTJG_OK) st = build_levels(ctx, n, 1, 2, M->rowptr, M->colind, M->diag, nullptr, M->up);
+                M->tickets32 = true;
+            }
             if (st != MTJG_OK) return st;
         }
     }
@@ -772,7 +781,7 @@ int precond_apply32(mtjg_precond *M, const float *b, float *x, const int *status
         e = cudaGetLastError();
         break;
     default: {  // ILU / ILUT: L y = b, then U x = y, on the FP32 factor
-        if (M->tile) {
+        if (M->tile && !M->tickets32) {
             e = tile_apply(ctx, M->tile, false, b, x, status, env_int("MTJG_SWEEP_SPIN", kSweepSpin, 0, 1 << 20));
             break;
         }
