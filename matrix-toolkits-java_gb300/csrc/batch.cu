@@ -45,14 +45,6 @@
 namespace mtjg {
 
 constexpr int kBatchBlock = 256;
-// resident CTAs per SM the batched CG is compiled for (its register cap).
-// Measured on GB300 (C4, FP64 / mixed): 3 (80 registers) 168.5 / 115.7 ms;
-// 4 (64 registers) 200.9 / 128.0 ms; 5: 238.6 / 152.8 ms -- the rows a
-// thread keeps in flight matter more than resident warps.
-#ifndef MTJG_BATCH_MINB
-#define MTJG_BATCH_MINB 3
-#endif
-constexpr int kBatchMinBlocks = MTJG_BATCH_MINB;
 constexpr int kProbeIters = 12;
 constexpr int kProbeSystems = 24;
 constexpr int kVecCandidates[] = {1, 2, 4, 8, 32};
@@ -539,7 +531,7 @@ __device__ void mixed_system(const BatchCg &a, int sys, Shared &sh, int &turn)
 
 // Teams of one size take the systems order[0 .. count) of that size.
 template <bool S, bool MIXED, bool TM>
-__global__ void __launch_bounds__(kBatchBlock, kBatchMinBlocks) k_batch_cg(BatchCg a)
+__global__ void __launch_bounds__(kBatchBlock, kBatchPerSm) k_batch_cg(BatchCg a)
 {
     __shared__ Shared sh;
     int turn = 0, rank = 0;
@@ -579,13 +571,14 @@ __global__ void __launch_bounds__(kBatchBlock, kBatchMinBlocks) k_batch_cg(Batch
 
 // One launch for the teams of `team` CTAs, on `stream`.
 template <bool S, bool MIXED>
-cudaError_t launch_teams(mtjg_ctx *ctx, const BatchCg &a, int team, cudaStream_t stream)
+cudaError_t launch_teams(mtjg_ctx *ctx, const BatchCg &a, int team, int most_per_sm, cudaStream_t stream)
 {
     auto k = team > 1 ? k_batch_cg<S, MIXED, true> : k_batch_cg<S, MIXED, false>;
     int per_sm = 0;
     cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kBatchBlock, 0);
     if (e != cudaSuccess) return e;
-    const int64_t room = std::max(team, ctx->num_sms * std::max(1, per_sm) / team * team);
+    per_sm = std::max(1, std::min(per_sm, most_per_sm));
+    const int64_t room = std::max(team, ctx->num_sms * per_sm / team * team);
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)std::max<int64_t>(1, std::min<int64_t>((int64_t)a.count * team, room)));
     cfg.blockDim = dim3(kBatchBlock);
@@ -602,7 +595,7 @@ cudaError_t launch_teams(mtjg_ctx *ctx, const BatchCg &a, int team, cudaStream_t
 }
 
 template <bool S, bool MIXED>
-cudaError_t launch_one(mtjg_ctx *ctx, BatchCg a, const int *counts)
+cudaError_t launch_one(mtjg_ctx *ctx, BatchCg a, const int *counts, int most_per_sm)
 {
     // each size of team on a stream of its own, between two events of the
     // context's stream; the largest first
@@ -627,7 +620,8 @@ cudaError_t launch_one(mtjg_ctx *ctx, BatchCg a, const int *counts)
             // the last size stays on the context's stream
             const bool side = --left > 0;
             if (side) e = cudaStreamWaitEvent(ctx->side[c], ctx->fork, 0);
-            if (e == cudaSuccess) e = launch_teams<S, MIXED>(ctx, b, 1 << (kTeamSizes - 1 - c), side ? ctx->side[c] : ctx->stream);
+            if (e == cudaSuccess) e = launch_teams<S, MIXED>(ctx, b, 1 << (kTeamSizes - 1 - c), most_per_sm,
+                                                            side ? ctx->side[c] : ctx->stream);
             if (e == cudaSuccess && side) e = cudaEventRecord(ctx->join[c], ctx->side[c]);
             forked[c] = side && e == cudaSuccess;
         }
@@ -654,27 +648,19 @@ int band(double v, const double *edges, int count)
 
 }  // namespace
 
-// CTAs of a system's team, as log2.  A share of 2048 rows or more is worth
-// the team's three barriers and rank-order sums per iteration (about 6000
-// cycles against 27,000 of FP64 work for 2048 rows of 19 entries).
-int batch_team(int64_t rows) { return rows >= 16384 ? 3 : rows >= 8192 ? 2 : rows >= 4096 ? 1 : 0; }
-
-void batch_teams(const int *sys_rows, std::vector<int> &order, int *counts)
+cudaError_t batch_launch(mtjg_ctx *ctx, const BatchCg &a, const int *sys_rows, const int *order, const int *counts,
+                         bool mixed)
 {
-    std::vector<int> by[kTeamSizes];
-    for (int s : order) by[kTeamSizes - 1 - batch_team((int64_t)sys_rows[s + 1] - sys_rows[s])].push_back(s);
-    order.clear();
-    for (int c = 0; c < kTeamSizes; ++c) {
-        counts[c] = (int)by[c].size();
-        order.insert(order.end(), by[c].begin(), by[c].end());
-    }
-}
-
-cudaError_t batch_launch(mtjg_ctx *ctx, const BatchCg &a, const int *counts, bool mixed)
-{
+    int kinds = 0, kind = 0;
+    for (int c = 0; c < kTeamSizes; ++c)
+        if (counts[c] > 0) ++kinds, kind = c;
+    // (launches beside each other fill the SMs' third place by themselves)
+    const int per_sm = kinds == 1 ? batch_per_sm(sys_rows, order, counts[kind], 1 << (kTeamSizes - 1 - kind), ctx->num_sms)
+                                  : kBatchPerSm;
     const bool strict = ctx->numerics == MTJG_NUMERICS_STRICT;
-    if (strict) return mixed ? launch_one<true, true>(ctx, a, counts) : launch_one<true, false>(ctx, a, counts);
-    return mixed ? launch_one<false, true>(ctx, a, counts) : launch_one<false, false>(ctx, a, counts);
+    auto go = [&](auto launch) { return launch(ctx, a, counts, per_sm); };
+    if (strict) return mixed ? go(launch_one<true, true>) : go(launch_one<true, false>);
+    return mixed ? go(launch_one<false, true>) : go(launch_one<false, false>);
 }
 
 // The class of a system: bands of its rows and of its entries per row.

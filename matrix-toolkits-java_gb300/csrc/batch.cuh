@@ -4,6 +4,7 @@
 #include <functional>
 #include <vector>
 
+#include "batch_plan.h"
 #include "phases.cuh"
 
 namespace mtjg {
@@ -32,13 +33,10 @@ struct BatchCg {
     MixCfg mix;
 };
 
-constexpr int kTeamSizes = 4;  // teams of 8, 4, 2 and 1 CTAs
-// Puts the systems of each team size together, largest teams first, each
-// keeping its order; counts[c]: systems of teams of 8 >> c CTAs.
-void batch_teams(const int *sys_rows, std::vector<int> &order, int *counts);
-// a.order as batch_teams left it (a.count is not read); a.ticket: kTeamSizes
-// counters, zero.
-cudaError_t batch_launch(mtjg_ctx *ctx, const BatchCg &a, const int *counts, bool mixed);
+// a.order and counts as batch_teams left them (order: the same on the host;
+// a.count is not read); a.ticket: kTeamSizes counters, zero.
+cudaError_t batch_launch(mtjg_ctx *ctx, const BatchCg &a, const int *sys_rows, const int *order, const int *counts,
+                         bool mixed);
 int batch_class(int64_t rows, int64_t nnz);
 int batch_tuned(int cls);
 // Lanes per row of each system (tuned per class, probing classes not seen

@@ -1579,7 +1579,7 @@ int run_batch(mtjg_solver *S, mtjg_csr *A, mtjg_result *res)
         cudaError_t e = cudaMemcpyAsync(S->b_order, placed.data(), sizeof(int) * placed.size(), cudaMemcpyHostToDevice,
                                         ctx->stream);
         if (e == cudaSuccess) e = cudaMemsetAsync(S->b_ticket, 0, sizeof(unsigned) * kTeamSizes, ctx->stream);
-        if (e == cudaSuccess) e = batch_launch(ctx, args, counts, S->mixed);
+        if (e == cudaSuccess) e = batch_launch(ctx, args, srow, placed.data(), counts, S->mixed);
         return e;
     };
     // lanes per row: STRICT sums every row in entry order (one lane)
