@@ -91,23 +91,62 @@ __device__ __forceinline__ void tri_range(const TriOp &op, int i, int &b, int &e
     e = op.range == 1 ? op.diag[i] : op.rp[i + 1];
 }
 
-// start[i] = 1 when row i begins a line: its last entry is not row i - 1
-__global__ void k_line_start(TriOp op, int *start)
+// An entry (i, c) of `op` and its mirror (c, i) in `other`
+__device__ __forceinline__ bool mirrored(const TriOp &op, const TriOp &other, int i, int &most)
 {
+    int b, e;
+    tri_range(op, i, b, e);
+    most = max(most, e - b);
+    bool all = true;
+    for (int k = b; k < e && e - b <= kLineK; ++k) {
+        int b2, e2;
+        tri_range(other, op.ci[k], b2, e2);
+        bool found = false;
+        for (int q = b2; q < e2 && e2 - b2 <= kLineK; ++q) found |= other.ci[q] == i;
+        all &= found;
+    }
+    return all;
+}
+
+// A row that begins a line: its last entry is not the row before
+__device__ __forceinline__ bool begins_line(const TriOp &op, int i)
+{
+    int b, e;
+    tri_range(op, i, b, e);
+    return !(e > b && op.ci[e - 1] == i - 1);
+}
+
+// count[0]: the longest row of both triangles, over kLineK where an entry has
+// no mirror in the other triangle; count[1]: the lines (0 and 0 before)
+__global__ void k_line_look(TriOp op, TriOp up, int *count)
+{
+    int most = 0, starts = 0;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < op.n; i += gridDim.x * blockDim.x) {
-        int b, e;
-        tri_range(op, i, b, e);
-        start[i] = !(e > b && op.ci[e - 1] == i - 1);
+        starts += begins_line(op, i);
+        const bool down = mirrored(op, up, i, most), above = mirrored(up, op, i, most);
+        if (!down || !above) most = max(most, kLineK + 1);
+    }
+    most = __reduce_max_sync(0xffffffffu, most);
+    starts = __reduce_add_sync(0xffffffffu, starts);
+    if ((threadIdx.x & 31) == 0) {
+        atomicMax(count, most);
+        atomicAdd(count + 1, starts);
     }
 }
 
-// line_of from the scan of start; each line's first row
-__global__ void k_line_of(int n, const int *start, const int *scan, int *line_of, int *first, int lines)
+__global__ void k_line_start(TriOp op, int *start)
+{
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < op.n; i += gridDim.x * blockDim.x)
+        start[i] = begins_line(op, i);
+}
+
+// line_of from the scan of start; each line's first row; pstart to 1
+__global__ void k_line_of(int n, const int *start, const int *scan, int *line_of, int *first, int *pstart, int lines)
 {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const int l = scan[i] + start[i] - 1;
         line_of[i] = l;
-        if (start[i]) first[l] = i;
+        if (start[i]) first[l] = i, pstart[l] = 1;
         if (i == 0) first[lines] = n;
     }
 }
@@ -125,23 +164,22 @@ __global__ void k_plane_start(TriOp op, const int *line_of, int *pstart)
     }
 }
 
-__global__ void k_fill(int n, int *p, int v)
-{
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) p[i] = v;
-}
-
-// each plane's first line, and the most lines of a plane
-__global__ void k_plane_first(int lines, const int *pstart, const int *scan, int *pfirst, int planes)
+// each plane's first line, the planes, and the most lines of a plane (0
+// before); scan[lines]: the planes
+__global__ void k_plane_first(int lines, const int *pstart, const int *scan, int *pfirst, int *planes)
 {
     for (int l = blockIdx.x * blockDim.x + threadIdx.x; l < lines; l += gridDim.x * blockDim.x) {
         if (pstart[l]) pfirst[scan[l]] = l;
-        if (l == 0) pfirst[planes] = lines;
+        if (l == 0) {
+            pfirst[scan[lines]] = lines;
+            *planes = scan[lines];
+        }
     }
 }
 
-__global__ void k_plane_long(int planes, const int *pfirst, int *longest)
+__global__ void k_plane_long(const int *planes, const int *pfirst, int *longest)
 {
-    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < planes; p += gridDim.x * blockDim.x)
+    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < *planes; p += gridDim.x * blockDim.x)
         atomicMax(longest, pfirst[p + 1] - pfirst[p]);
 }
 
@@ -217,7 +255,8 @@ __global__ void k_line_deps(TriOp op, int lines, const int *line_of, const int *
     }
 }
 
-// The lowest offsets, in one block, and each part's first and last step.
+// The lowest offsets, in one block, each part's first and last step, and the
+// parts' places one behind the other.
 // Plane after plane: a line starts after the plane's line before it (a scan
 // of the maps t -> max(b, t + a)) and after what it reads in earlier planes.
 // Then rounds over all lines until none moves, which cover what the scan left
@@ -230,13 +269,15 @@ constexpr int kOffsetBlock = 1024;
 constexpr int kScanPlanes = 2048;
 __global__ void __launch_bounds__(kOffsetBlock) k_line_offsets(int lines, int planes, const int *pfirst,
                                                                const int2 *dep, const int *first, const int *part_of,
-                                                               int *off, int *lo, int *hi, int *bad)
+                                                               int *off, int parts, int *lo, int *hi, int *part_step,
+                                                               int *bad)
 {
     extern __shared__ int s_off[];
     __shared__ int s_a[kOffsetBlock / 32], s_b[kOffsetBlock / 32];
     constexpr int kNone = -0x20000000;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     for (int l = tid; l < lines; l += kOffsetBlock) s_off[l] = 0;
+    for (int p = tid; p < parts; p += kOffsetBlock) lo[p] = 0x7fffffff, hi[p] = -1;
     __syncthreads();
     for (int p = 0; p < planes && planes <= kScanPlanes; ++p) {
         const int l0 = pfirst[p], l1 = pfirst[p + 1];
@@ -302,40 +343,32 @@ __global__ void __launch_bounds__(kOffsetBlock) k_line_offsets(int lines, int pl
         atomicMin(lo + part_of[l], v);
         atomicMax(hi + part_of[l], v + first[l + 1] - first[l] - 1);
     }
+    __syncthreads();
+    if (tid == 0) {  // (a plan of more steps than an int holds is refused)
+        long long step = 0;
+        for (int p = 0; p < parts; ++p) {
+            part_step[p] = (int)step;
+            const int l = __ldcg(lo + p), h = __ldcg(hi + p);
+            step = min(step + max(0, h - l + 1), 0x7fffffffLL);
+        }
+        part_step[parts] = (int)step;
+    }
 }
 
-// each row's position, and the row at each position (row is -1 before)
+// each row's position, the row at each position (row is -1 before), and the
+// parts' steps into the plan's own array
 __global__ void k_line_place(int n, int lanes, const int *line_of, const int *first, const int *part_of,
-                             const int *lane_of, const int *off, const int *part_min, const int *part_step, int *pos,
-                             int *row)
+                             const int *lane_of, const int *off, const int *part_min, int parts, const int *part_step,
+                             int *pos, int *row, int *plan_step)
 {
+    if (blockIdx.x == 0)
+        for (int p = threadIdx.x; p <= parts; p += blockDim.x) plan_step[p] = part_step[p];
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const int l = line_of[i], p = part_of[l];
         const int at = (part_step[p] + off[l] + (i - first[l]) - part_min[p]) * lanes + lane_of[l];
         pos[i] = at;
         row[at] = i;
     }
-}
-
-// *bad = 1 unless every entry (i, c) of `op` has its mirror (c, i) in `other`;
-// kmax: the longest row (over kLineK rules the plan out)
-__global__ void k_mirrored(TriOp op, TriOp other, int *kmax, int *bad)
-{
-    int km = 0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < op.n; i += gridDim.x * blockDim.x) {
-        int b, e;
-        tri_range(op, i, b, e);
-        km = max(km, e - b);
-        for (int k = b; k < e && e - b <= kLineK; ++k) {
-            int b2, e2;
-            tri_range(other, op.ci[k], b2, e2);
-            bool found = false;
-            for (int q = b2; q < e2 && e2 - b2 <= kLineK; ++q) found |= other.ci[q] == i;
-            if (!found) *bad = 1;
-        }
-    }
-    for (int off = 16; off > 0; off >>= 1) km = max(km, __shfl_down_sync(0xffffffffu, km, off));
-    if ((threadIdx.x & 31) == 0) atomicMax(kmax, km);
 }
 
 // The part that holds a step: part_step is ascending (binary search).
@@ -352,9 +385,11 @@ __device__ __forceinline__ int part_at(const int *part_step, int parts, int step
 
 // The entry codes of every position (without a row every code is the zero's)
 // and, with `rem`, the remote entries of each step: rem_max places a step,
-// (-1, 0) before; cursor counts a step's entries, beyond rem_max too.
+// (-1, 0) before; cursor counts a step's entries, and *longest is raised to
+// the count of a step that has more.
 template <class V>
-__global__ void k_line_codes(TriOp op, TilePlan tp, unsigned char *rec, int *cursor, int2 *rem, int rem_max)
+__global__ void k_line_codes(TriOp op, TilePlan tp, unsigned char *rec, int *cursor, int2 *rem, int rem_max,
+                             int *longest)
 {
     const int T = tp.lanes, K = tp.kmax, bytes = line_record<V>(K, T);
     for (int at = blockIdx.x * blockDim.x + threadIdx.x; at < tp.steps * T; at += gridDim.x * blockDim.x) {
@@ -377,6 +412,7 @@ __global__ void k_line_codes(TriOp op, TilePlan tp, unsigned char *rec, int *cur
                     if (rem) {
                         const int q = atomicAdd(cursor + step, 1);
                         if (q < rem_max) rem[(size_t)step * rem_max + q] = make_int2(c, k * T + lane);
+                        else atomicMax(longest, q + 1);
                     }
                 }
             }
@@ -825,9 +861,6 @@ cudaError_t tile_apply(mtjg_ctx *ctx, const TilePair *t, bool strict, const floa
 static void free_plan(TilePlan *&tp)
 {
     if (!tp) return;
-    cudaFree(tp->part_step);
-    cudaFree(tp->pos);
-    cudaFree(tp->row);
     cudaFree(tp->b64);
     cudaFree(tp->b32);
     delete tp;
@@ -838,11 +871,8 @@ void free_tiles_of(TilePair *&t)
 {
     if (!t) return;
     if (t->owns_plan) free_plan(t->plan);
-    for (TileOp &op : t->op) {
-        cudaFree(op.rec64);
-        cudaFree(op.rec32);
-        cudaFree(op.rem);
-    }
+    cudaFree(t->mem);
+    for (TileOp &op : t->op) cudaFree(op.rec32);
     delete t;
     t = nullptr;
 }
@@ -873,11 +903,9 @@ static int tile_plan(mtjg_ctx *ctx, const TriOp &op, const TriOp &up, TilePlan *
         return MTJG_OK;
     TilePlan *tp = new TilePlan();
     tp->n = n;
-    int *work = nullptr, *lw = nullptr, *pw = nullptr;
+    int *work = nullptr;
     auto done = [&](int st, bool keep) {
         cudaFree(work);
-        cudaFree(lw);
-        cudaFree(pw);
         if (keep) *out = tp;
         else free_plan(tp);
         return st;
@@ -889,43 +917,51 @@ static int tile_plan(mtjg_ctx *ctx, const TriOp &op, const TriOp &up, TilePlan *
     } while (0)
     cudaStream_t q = ctx->stream;
     const int g = grid_rows(ctx, n);
-    LP_CUDA(cudaMalloc(&work, sizeof(int) * (3 * (size_t)n + 2 + 4)));
-    int *start = work, *scan = start + n, *line_of = scan + n + 1, *scalars = line_of + n;
-    // scalars: longest row, lines of the longest plane, 1 for lines without offsets, 1 unless mirrored
-    LP_CUDA(cudaMemsetAsync(scalars, 0, sizeof(int) * 4, q));
-    k_line_start<<<g, kBlock, 0, q>>>(op, start);
-    k_mirrored<<<g, kBlock, 0, q>>>(op, up, scalars, scalars + 3);
-    k_mirrored<<<g, kBlock, 0, q>>>(up, op, scalars, scalars + 3);
-    ctx->launches += 3;
-    int st = exclusive_scan(ctx, start, scan, n);
-    if (st != MTJG_OK) return done(st, false);
-    int lines = 0, sc[4] = {};
-    LP_CUDA(cudaMemcpyAsync(&lines, scan + n, sizeof(int), cudaMemcpyDeviceToHost, q));
-    LP_CUDA(cudaMemcpyAsync(sc, scalars, sizeof(sc), cudaMemcpyDeviceToHost, q));
+    // Planning costs allocations, launches and waits beside its kernels, and on
+    // a small or refused factor they are all there is.  First the pattern by
+    // itself, before anything is allocated (setMatrix of a permuted 20^3 grid,
+    // refused: 943 us with levels alone, 995 with two allocations before the
+    // refusal, 977 so); then one allocation of scratch, one of the plan, one of
+    // both sweeps' records, and four waits in all (four rows of four, ILU: 312 us
+    // with levels alone, 395 with 15 allocations and nine waits, 274 so; ICC 329,
+    // 471, 390).
+    int *look = ctx->d_flag + 2, sc[2] = {};
+    LP_CUDA(cudaMemsetAsync(look, 0, sizeof(sc), q));
+    k_line_look<<<g, kBlock, 0, q>>>(op, up, look);
+    ctx->launches++;
+    LP_CUDA(cudaMemcpyAsync(sc, look, sizeof(sc), cudaMemcpyDeviceToHost, q));
     LP_CUDA(cudaStreamSynchronize(q));
+    const int lines = sc[1];
     tp->kmax = sc[0] == 1 ? 2 : sc[0];
-    if (tp->kmax < 2 || tp->kmax > kLineK || sc[3] || (int64_t)lines * kMinLine > n) return done(MTJG_OK, false);
-    // what each line reads, first row of each line, plane starts and their
-    // scan, first line of each plane, part, lane and offset
-    LP_CUDA(cudaMalloc(&lw, sizeof(int) * ((7 + 2 * kLineK) * (size_t)lines + 4)));
-    int2 *dep = reinterpret_cast<int2 *>(lw);
-    int *first = lw + 2 * kLineK * (size_t)lines, *pstart = first + lines + 1, *pscan = pstart + lines, *pfirst = pscan + lines + 1;
-    int *part_of = pfirst + lines + 1, *lane_of = part_of + lines, *off = lane_of + lines;
+    if (tp->kmax < 2 || tp->kmax > kLineK || (int64_t)lines * kMinLine > n) return done(MTJG_OK, false);
+    // one allocation: what each line reads; per row the start of a line, the
+    // line and the starts' scan; counts; per line its first row, the start of a
+    // plane and its scan, the planes' first lines, part, lane and offset; per
+    // part its first step, last step and place; the scans' scratch
+    const size_t L = (size_t)lines, P0 = (size_t)ctx->num_sms;
+    LP_CUDA(cudaMalloc(&work, sizeof(int) * (2 * kLineK * L + 3 * (size_t)n + 1 + 3 + 7 * L + 3 + 3 * P0 + 1 +
+                                             (size_t)scan_scratch(n))));
+    int2 *dep = reinterpret_cast<int2 *>(work);
+    int *start = work + 2 * kLineK * L, *line_of = start + n, *scan = line_of + n;
+    // planes, lines of the longest plane, 1 for lines without offsets
+    int *scalars = scan + n + 1;
+    int *first = scalars + 3, *pstart = first + L + 1, *pscan = pstart + L, *pfirst = pscan + L + 1;
+    int *part_of = pfirst + L + 1, *lane_of = part_of + L, *off = lane_of + L;
+    int *pw = off + L, *scratch = pw + 3 * P0 + 1;
+    LP_CUDA(cudaMemsetAsync(scalars, 0, sizeof(int) * 3, q));
+    k_line_start<<<g, kBlock, 0, q>>>(op, start);
+    ctx->launches++;
+    LP_CUDA(exclusive_scan_async(ctx, start, scan, n, scratch));
     const int gl = grid_rows(ctx, lines);
-    k_line_of<<<g, kBlock, 0, q>>>(n, start, scan, line_of, first, lines);
-    k_fill<<<gl, kBlock, 0, q>>>(lines, pstart, 1);
+    k_line_of<<<g, kBlock, 0, q>>>(n, start, scan, line_of, first, pstart, lines);
     k_plane_start<<<g, kBlock, 0, q>>>(op, line_of, pstart);
-    ctx->launches += 3;
-    st = exclusive_scan(ctx, pstart, pscan, lines);
-    if (st != MTJG_OK) return done(st, false);
-    int planes = 0, longest = 0;
-    LP_CUDA(cudaMemcpyAsync(&planes, pscan + lines, sizeof(int), cudaMemcpyDeviceToHost, q));
+    LP_CUDA(exclusive_scan_async(ctx, pstart, pscan, lines, scratch));
+    k_plane_first<<<gl, kBlock, 0, q>>>(lines, pstart, pscan, pfirst, scalars);
+    k_plane_long<<<gl, kBlock, 0, q>>>(scalars, pfirst, scalars + 1);
+    ctx->launches += 4;
+    LP_CUDA(cudaMemcpyAsync(sc, scalars, sizeof(int) * 2, cudaMemcpyDeviceToHost, q));
     LP_CUDA(cudaStreamSynchronize(q));
-    k_plane_first<<<gl, kBlock, 0, q>>>(lines, pstart, pscan, pfirst, planes);
-    k_plane_long<<<grid_rows(ctx, planes), kBlock, 0, q>>>(planes, pfirst, scalars + 1);
-    ctx->launches += 2;
-    LP_CUDA(cudaMemcpyAsync(&longest, scalars + 1, sizeof(int), cudaMemcpyDeviceToHost, q));
-    LP_CUDA(cudaStreamSynchronize(q));
+    const int planes = sc[0], longest = sc[1];
     int tq = 0, ntq = 0, best = 0;
     for (int T = 128; T <= 256 && !tp->parts; T *= 2)
         for (int a = 1; a <= T; a *= 2) {
@@ -948,39 +984,29 @@ static int tile_plan(mtjg_ctx *ctx, const TriOp &op, const TriOp &up, TilePlan *
     // worth finding
     const int64_t likely = (int64_t)P * (n / lines - 2) + (int64_t)(P / ntq) * longest + (int64_t)ntq * planes;
     if (likely * T > 2 * (2 * (int64_t)n + 65536)) return done(MTJG_OK, false);
-    LP_CUDA(cudaMalloc(&pw, sizeof(int) * 2 * (size_t)P));
-    LP_CUDA(cudaMalloc(&tp->part_step, sizeof(int) * (size_t)(P + 1)));
-    LP_CUDA(cudaMalloc(&tp->pos, sizeof(int) * (size_t)n));
+    int *part_step = pw + 2 * (size_t)P;
     k_line_tile<<<gl, kBlock, 0, q>>>(lines, pstart, pscan, pfirst, tq, T / tq, ntq, part_of, lane_of);
-    k_fill<<<1, kBlock, 0, q>>>(P, pw, 0x7fffffff);
-    k_fill<<<1, kBlock, 0, q>>>(P, pw + P, -1);
     k_line_deps<<<(lines + 7) / 8, kBlock, 0, q>>>(op, lines, line_of, first, dep, scalars + 2);
     LP_CUDA(cudaFuncSetAttribute(k_line_offsets, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - 1024));
     k_line_offsets<<<1, kOffsetBlock, sizeof(int) * (size_t)lines, q>>>(lines, planes, pfirst, dep, first, part_of, off,
-                                                                        pw, pw + P, scalars + 2);
-    ctx->launches += 5;
-    std::vector<int> span(2 * (size_t)P), step((size_t)P + 1, 0);
-    LP_CUDA(cudaMemcpyAsync(span.data(), pw, sizeof(int) * 2 * (size_t)P, cudaMemcpyDeviceToHost, q));
-    LP_CUDA(cudaMemcpyAsync(sc, scalars, sizeof(sc), cudaMemcpyDeviceToHost, q));
+                                                                        P, pw, pw + P, part_step, scalars + 2);
+    ctx->launches += 3;
+    LP_CUDA(cudaMemcpyAsync(sc, scalars + 2, sizeof(int), cudaMemcpyDeviceToHost, q));
+    LP_CUDA(cudaMemcpyAsync(sc + 1, part_step + P, sizeof(int), cudaMemcpyDeviceToHost, q));
     LP_CUDA(cudaStreamSynchronize(q));
-    if (sc[2]) return done(MTJG_OK, false);
-    int64_t steps = 0;
-    for (int p = 0; p < P; ++p) {
-        const int lo = span[(size_t)p], hi = span[(size_t)(P + p)];
-        steps += hi >= lo ? hi - lo + 1 : 0;
-        if (steps * T > 2 * (int64_t)n + 65536) return done(MTJG_OK, false);
-        step[(size_t)p + 1] = (int)steps;
-    }
-    tp->steps = (int)steps;
-    const size_t count = (size_t)steps * T;
-    LP_CUDA(cudaMemcpyAsync(tp->part_step, step.data(), sizeof(int) * (size_t)(P + 1), cudaMemcpyHostToDevice, q));
-    LP_CUDA(cudaMalloc(&tp->row, sizeof(int) * count));
-    LP_CUDA(cudaMemsetAsync(tp->row, 0xff, sizeof(int) * count, q));
-    k_line_place<<<g, kBlock, 0, q>>>(n, T, line_of, first, part_of, lane_of, off, pw, tp->part_step, tp->pos, tp->row);
-    ctx->launches++;
-    LP_CUDA(cudaMalloc(&tp->b64, sizeof(double) * 3 * count));
+    tp->steps = sc[1];
+    if (sc[0] || (int64_t)tp->steps * T > 2 * (int64_t)n + 65536) return done(MTJG_OK, false);
+    const size_t count = (size_t)tp->steps * T;
+    LP_CUDA(cudaMalloc(&tp->b64, sizeof(double) * 3 * count + sizeof(int) * (count + (size_t)n + (size_t)P + 1)));
     tp->y64 = tp->b64 + count;
     tp->x64 = tp->y64 + count;
+    tp->row = reinterpret_cast<int *>(tp->x64 + count);
+    tp->pos = tp->row + count;
+    tp->part_step = tp->pos + n;
+    LP_CUDA(cudaMemsetAsync(tp->row, 0xff, sizeof(int) * count, q));
+    k_line_place<<<g, kBlock, 0, q>>>(n, T, line_of, first, part_of, lane_of, off, pw, P, part_step, tp->pos, tp->row,
+                                      tp->part_step);
+    ctx->launches++;
     // a launch that has nothing to do (a status other than running) tells
     // whether the device takes this cooperative grid
     static_assert(ST_RUNNING != -1, "the trial launch's status");
@@ -993,48 +1019,44 @@ static int tile_plan(mtjg_ctx *ctx, const TriOp &op, const TriOp &up, TilePlan *
         return done(MTJG_OK, false);
     }
     LP_CUDA(e);
-    LP_CUDA(cudaStreamSynchronize(q));
     return done(MTJG_OK, true);
 }
 #undef LP_CUDA
 
-// A sweep's entry codes and the lists of what it reads from other parts: 32
+// The sweeps' entry codes and the lists of what they read from other parts: 32
 // places a step (a tile of 8 x 16 lines of a grid needs at most 24), or as
 // many as the longest needs.
-__global__ void k_most(int n, const int *v, int *most)
+static int tile_ops(mtjg_ctx *ctx, TilePair *t, const TriOp &lo, const TriOp &up)
 {
-    int m = 0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) m = max(m, v[i]);
-    for (int off = 16; off > 0; off >>= 1) m = max(m, __shfl_down_sync(0xffffffffu, m, off));
-    if ((threadIdx.x & 31) == 0) atomicMax(most, m);
-}
-
-static int tile_op(mtjg_ctx *ctx, const TilePlan *tp, const TriOp &op, TileOp &out)
-{
-    out.mode = op.mode;
+    const TilePlan *tp = t->plan;
     cudaStream_t q = ctx->stream;
-    const int S = tp->steps, g = grid_rows(ctx, (int64_t)S * tp->lanes);
-    int *cursor = nullptr;
-    MTJG_CUDA(cudaMalloc(&out.rec64, (size_t)S * line_record<double>(tp->kmax, tp->lanes)));
-    MTJG_CUDA(cudaMalloc(&cursor, sizeof(int) * (size_t)(S + 1)));
-    cudaError_t e = cudaSuccess;
+    const size_t S = (size_t)tp->steps, rec = S * line_record<double>(tp->kmax, tp->lanes);
+    const int g = grid_rows(ctx, (int64_t)S * tp->lanes);
+    // the longest lists and the steps' counts, in a vector that no sweep uses now
+    int *longest = reinterpret_cast<int *>(tp->y64), h[2] = {};
     int most = 32;
     do {
-        out.rem_max = most;
-        cudaFree(out.rem);
-        out.rem = nullptr;
-        const size_t bytes = sizeof(int2) * (size_t)S * most;
-        if ((e = cudaMalloc(&out.rem, bytes)) != cudaSuccess) break;
-        cudaMemsetAsync(out.rem, 0xff, bytes, q);
-        cudaMemsetAsync(cursor, 0, sizeof(int) * (size_t)(S + 1), q);
-        k_line_codes<double><<<g, kBlock, 0, q>>>(op, *tp, out.rec64, cursor, (int2 *)out.rem, most);
-        k_most<<<grid_rows(ctx, S), kBlock, 0, q>>>(S, cursor, cursor + S);
-        ctx->launches += 2;
-        e = cudaMemcpyAsync(&most, cursor + S, sizeof(int), cudaMemcpyDeviceToHost, q);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(q);
-    } while (e == cudaSuccess && most > out.rem_max);
-    cudaFree(cursor);
-    if (e != cudaSuccess) return cuda_fail(e, "sweep plan");
+        const size_t rem = sizeof(int2) * S * most;
+        cudaFree(t->mem);
+        t->mem = nullptr;
+        MTJG_CUDA(cudaMalloc(&t->mem, 2 * (rec + rem)));
+        MTJG_CUDA(cudaMemsetAsync(t->mem + 2 * rec, 0xff, 2 * rem, q));
+        MTJG_CUDA(cudaMemsetAsync(longest, 0, sizeof(int) * (2 * S + 2), q));
+        for (int w = 0; w < 2; ++w) {
+            TileOp &o = t->op[w];
+            int *cursor = longest + 2 + w * S;
+            o.mode = w ? up.mode : lo.mode;
+            o.rec64 = t->mem + w * rec;
+            o.rem = reinterpret_cast<int *>(t->mem + 2 * rec + w * rem);
+            o.rem_max = most;
+            k_line_codes<double><<<g, kBlock, 0, q>>>(w ? up : lo, *tp, o.rec64, cursor, (int2 *)o.rem, most,
+                                                     longest + w);
+            ctx->launches++;
+        }
+        MTJG_CUDA(cudaMemcpyAsync(h, longest, sizeof(h), cudaMemcpyDeviceToHost, q));
+        MTJG_CUDA(cudaStreamSynchronize(q));
+        h[0] = std::max(h[0], h[1]);
+    } while (h[0] > most && (most = h[0]));
     return MTJG_OK;
 }
 
@@ -1046,10 +1068,7 @@ int tile_pair(mtjg_ctx *ctx, const TriOp &lo, const TriOp &up, TilePlan *plan, T
     t->plan = plan;
     int st = MTJG_OK;
     if (!plan) st = tile_plan(ctx, lo, up, &t->plan);
-    if (st == MTJG_OK && t->plan) {
-        st = tile_op(ctx, t->plan, lo, t->op[0]);
-        if (st == MTJG_OK) st = tile_op(ctx, t->plan, up, t->op[1]);
-    }
+    if (st == MTJG_OK && t->plan) st = tile_ops(ctx, t, lo, up);
     if (st != MTJG_OK || !t->plan) free_tiles_of(t);
     else *out = t;
     if (st == MTJG_ERR_OUT_OF_MEMORY) {  // the level schedules take a tenth of the memory
@@ -1191,7 +1210,7 @@ int tile_values(mtjg_ctx *ctx, TilePair *t, int which, const TriOp &op, const fl
         const size_t bytes = (size_t)tp->steps * line_record<float>(tp->kmax, tp->lanes);
         MTJG_CUDA(cudaMalloc(&to.rec32, bytes));
         k_line_codes<float><<<grid_rows(ctx, (int64_t)count), kBlock, 0, ctx->stream>>>(
-            op, *tp, to.rec32, nullptr, nullptr, 0);
+            op, *tp, to.rec32, nullptr, nullptr, 0, nullptr);
         ctx->launches++;
     }
     k_line_values<float><<<grid_rows(ctx, (int64_t)count), kBlock, 0, ctx->stream>>>(op, *tp, to.rec32, v, diagv);

@@ -21,10 +21,11 @@ struct TilePlan {
     int n = 0, kmax = 0;      // rows, entries of the longest row of either triangle
     int parts = 0, lanes = 0;
     int steps = 0;            // steps of all parts
-    int *part_step = nullptr; // device [parts + 1]: first step of each part
-    int *pos = nullptr;       // device [n]: position of each row
-    int *row = nullptr;       // device [steps * lanes]: row at each position, -1 for none
+    // one device allocation, at b64:
     double *b64 = nullptr, *y64 = nullptr, *x64 = nullptr;  // vectors in plan order
+    int *row = nullptr;       // [steps * lanes]: row at each position, -1 for none
+    int *pos = nullptr;       // [n]: position of each row
+    int *part_step = nullptr; // [parts + 1]: first step of each part
     float *b32 = nullptr, *y32 = nullptr, *x32 = nullptr;
 };
 
@@ -36,7 +37,7 @@ struct TilePlan {
 struct TileOp {
     int mode = 0;
     unsigned char *rec64 = nullptr, *rec32 = nullptr;
-    int *rem = nullptr;       // device [steps][rem_max][2]
+    int *rem = nullptr;       // [steps][rem_max][2]
     int rem_max = 0;
 };
 
@@ -44,6 +45,7 @@ struct TileOp {
 struct TilePair {
     TilePlan *plan = nullptr;
     bool owns_plan = true;
+    unsigned char *mem = nullptr;  // device: both ops' rec64 and rem
     TileOp op[2];
 };
 

@@ -243,21 +243,26 @@ __global__ void k_scan_apply(const int *in, int n, const int *chunk_off, int *ou
     if (c == (int)gridDim.x - 1 && threadIdx.x == 0) out[n] = chunk_off[gridDim.x];
 }
 
+int scan_scratch(int n) { return (n + kScanChunk - 1) / kScanChunk + 1; }
+
+cudaError_t exclusive_scan_async(mtjg_ctx *ctx, const int *in, int *out, int n, int *scratch)
+{
+    if (n == 0) return cudaMemsetAsync(out, 0, sizeof(int), ctx->stream);
+    const int nc = (n + kScanChunk - 1) / kScanChunk;
+    k_scan_chunks<<<nc, kBlock, 0, ctx->stream>>>(in, n, scratch);
+    k_scan_top<<<1, kBlock, 0, ctx->stream>>>(scratch, nc);
+    k_scan_apply<<<nc, kBlock, 0, ctx->stream>>>(in, n, scratch, out);
+    ctx->launches += 3;
+    return cudaGetLastError();
+}
+
 int exclusive_scan(mtjg_ctx *ctx, const int *in, int *out, int n)
 {
-    if (n == 0) {
-        MTJG_CUDA(cudaMemsetAsync(out, 0, sizeof(int), ctx->stream));
-        return MTJG_OK;
-    }
-    int nc = (n + kScanChunk - 1) / kScanChunk;
-    int *cs = nullptr;
-    MTJG_CUDA(cudaMalloc(&cs, sizeof(int) * (nc + 1)));
-    k_scan_chunks<<<nc, kBlock, 0, ctx->stream>>>(in, n, cs);
-    k_scan_top<<<1, kBlock, 0, ctx->stream>>>(cs, nc);
-    k_scan_apply<<<nc, kBlock, 0, ctx->stream>>>(in, n, cs, out);
-    ctx->launches += 3;
-    cudaError_t e = cudaStreamSynchronize(ctx->stream);
-    cudaFree(cs);
+    int *scratch = nullptr;
+    MTJG_CUDA(cudaMalloc(&scratch, sizeof(int) * (size_t)scan_scratch(n)));
+    cudaError_t e = exclusive_scan_async(ctx, in, out, n, scratch);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+    cudaFree(scratch);
     if (e != cudaSuccess) return cuda_fail(e, "exclusive_scan");
     return MTJG_OK;
 }

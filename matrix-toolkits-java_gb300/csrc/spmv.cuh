@@ -779,6 +779,9 @@ int upload_tiles(TileSet &ts, const std::vector<int> &tile_row, const std::vecto
 void free_tiles(TileSet &ts);
 // Device exclusive scan of n ints into out[0..n] (out[n] = total).
 int exclusive_scan(mtjg_ctx *ctx, const int *in, int *out, int n);
+// the same without a wait; scratch: scan_scratch(n) ints on the device
+int scan_scratch(int n);
+cudaError_t exclusive_scan_async(mtjg_ctx *ctx, const int *in, int *out, int n, int *scratch);
 // Device transpose of selected entries of a CSR: mode 0 = all entries,
 // mode 1 = strictly upper entries (column > row), mode 2 = strictly lower.
 // Rows of the result list their entries in ascending source row order; the
