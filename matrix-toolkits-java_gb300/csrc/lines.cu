@@ -25,6 +25,7 @@
 // levels only, and all CTAs run at once (a cooperative launch), so the sweep
 // cannot deadlock: the lowest unfinished level is always free to run.
 #include <algorithm>
+#include <type_traits>
 #include <vector>
 
 #include "lines.cuh"
@@ -82,6 +83,21 @@ constexpr int line_smem(int kmax, int lanes)
 {
     return (MODE == 6 ? 2 : 1) * line_slots<V>(kmax, lanes) +
            LinePipe<V>::kSlots * (mode_record<V, MODE>(kmax, lanes) + lanes * (int)sizeof(V));
+}
+
+// What fits a CTA (227 KB, of which the kernel's own variables take little):
+// a plan serves both precisions, so four entries of 256 lanes (FP32: 254 KB)
+// are never planned; the pivots' sweep of 256 lanes holds two entries (280 KB
+// for three), and a factor of more takes the elimination by levels.
+constexpr int kLineSmem = 226 * 1024;
+constexpr bool line_plan_fits(int kmax, int lanes)
+{
+    return line_smem<double>(kmax, lanes) <= kLineSmem && line_smem<float>(kmax, lanes) <= kLineSmem;
+}
+template <int MODE>
+constexpr bool line_fits(int kmax, int lanes)
+{
+    return MODE == 6 ? line_smem<double, 6>(kmax, lanes) <= kLineSmem : line_plan_fits(kmax, lanes);
 }
 
 // ------------------------------------------------------------ the plan
@@ -781,17 +797,18 @@ template <bool S, int MODE, class V>
 cudaError_t launch_k(mtjg_ctx *ctx, const TilePlan *tp, const TileOp &op, const V *b, V *x, const int *status, int spin,
                      int *pivot0 = nullptr)
 {
-    const bool wide = tp->lanes == 256;
+    const auto go = [&](auto kmax) {
+        constexpr int K = decltype(kmax)::value;
+        if constexpr (line_fits<MODE>(K, 256)) {
+            if (tp->lanes == 256) return launch_line<S, MODE, K, 256, V>(ctx, tp, op, b, x, status, spin, pivot0);
+        }
+        if (tp->lanes != 128) return cudaErrorInvalidConfiguration;  // (tile_plan and tile_ilu ask line_fits)
+        return launch_line<S, MODE, K, 128, V>(ctx, tp, op, b, x, status, spin, pivot0);
+    };
     switch (tp->kmax) {
-    case 2:
-        return wide ? launch_line<S, MODE, 2, 256, V>(ctx, tp, op, b, x, status, spin, pivot0)
-                    : launch_line<S, MODE, 2, 128, V>(ctx, tp, op, b, x, status, spin, pivot0);
-    case 3:
-        return wide ? launch_line<S, MODE, 3, 256, V>(ctx, tp, op, b, x, status, spin, pivot0)
-                    : launch_line<S, MODE, 3, 128, V>(ctx, tp, op, b, x, status, spin, pivot0);
-    default:
-        return wide ? launch_line<S, MODE, 4, 256, V>(ctx, tp, op, b, x, status, spin, pivot0)
-                    : launch_line<S, MODE, 4, 128, V>(ctx, tp, op, b, x, status, spin, pivot0);
+    case 2: return go(std::integral_constant<int, 2>{});
+    case 3: return go(std::integral_constant<int, 3>{});
+    default: return go(std::integral_constant<int, 4>{});
     }
 }
 
@@ -975,8 +992,7 @@ static int tile_plan(mtjg_ctx *ctx, const TriOp &op, const TriOp &up, TilePlan *
         }
     int optin = 0;
     LP_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
-    if (!tp->parts || (int64_t)lines * 4 + 1024 > optin || line_smem<double>(tp->kmax, tp->lanes) + 1024 > optin ||
-        line_smem<float>(tp->kmax, tp->lanes) + 1024 > optin)
+    if (!tp->parts || (int64_t)lines * 4 + 1024 > optin || !line_plan_fits(tp->kmax, tp->lanes))
         return done(MTJG_OK, false);
     const int P = tp->parts, T = tp->lanes;
     // a grid's steps (a part of q by p lines of L rows takes L + q + p - 2):
@@ -1146,10 +1162,8 @@ int tile_ilu(mtjg_ctx *ctx, TilePair *t, const TriOp &lo, double *data, bool *fa
 {
     *factored = false;
     const TilePlan *tp = t->plan;
-    int optin = 0;
-    MTJG_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
     const int64_t count = (int64_t)tp->steps * tp->lanes;
-    if (line_smem<double, 6>(tp->kmax, tp->lanes) + 1024 > optin || !pivot_pairs_fit(count)) return MTJG_OK;
+    if (!line_fits<6>(tp->kmax, tp->lanes) || !pivot_pairs_fit(count)) return MTJG_OK;
     cudaStream_t q = ctx->stream;
     const size_t bytes = (size_t)tp->steps * mode_record<double, 6>(tp->kmax, tp->lanes);
     unsigned char *rec = nullptr;
