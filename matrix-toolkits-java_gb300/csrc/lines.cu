@@ -496,13 +496,20 @@ __global__ void k_tile_out(int n, const int *pos, const V *xp, V *x, const int *
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) x[i] = xp[pos[i]];
 }
 
-// a / d from y = RN(1 / d) by one residual correction (two in STRICT and
-// FP32): P. Markstein, "Computation of elementary functions on the IBM RISC
-// System/6000 processor", IBM J. Res. Dev. 34 (1990): with y the rounded
-// reciprocal, a faithful quotient corrected by its exact residual is the
-// rounded quotient.  The first correction makes q faithful (and the rounded
-// quotient but for about one operand pair in 2^52), the second settles it.
-// Out of the range where every intermediate is normal: a real division.
+// a / d from y = RN(1 / d) by one residual correction, the rounded quotient
+// (P. Markstein, "Computation of elementary functions on the IBM RISC
+// System/6000 processor", IBM J. Res. Dev. 34 (1990), for the method).  With
+// d' in [1, 2) the significand of d, 1 - d y is at most 2^-54 d'.  Before its
+// last rounding, q0 + (a - q0 d) y differs from a / d by (a / d - q0)(1 - d y).
+// a / d lies at least 1 / (2 d) = 2^-53 / d' units off every midpoint between
+// two doubles (d as an integer of 53 bits).  Only where it lies within 1.5 *
+// 2^-53 units of one could the last rounding differ, and there a y is less than
+// a whole unit off the midpoint, so q0 is one of its two neighbours, half a unit
+// away: the difference is at most 2^-54 d' / 2, which is less than 2^-53 / d' for
+// every d' < 2 (d = 2^53 - 1, where the bounds meet, included; the quotients
+// nearest to midpoints are in tests/test_gpu_line_division.py).  STRICT and FP32
+// take a second correction.  Out of the range where every intermediate is
+// normal: a real division.
 // a real division, kept out of line: inlined, its steps were computed ahead
 // of the test on every row
 __device__ __noinline__ double full_div(double a, double d) { return a / d; }
