@@ -121,8 +121,9 @@ __device__ __forceinline__ void team_rows(const BatchCg &a, int sys, int &r0, in
 
 // row i of A (x gathered), summed by VEC lanes in entry order per lane and a
 // fixed butterfly; every lane of the group returns the sum.  The matrix is
-// read-only for the launch (read-only path); x was written by this CTA
-// earlier in the launch, so it is read with coherent loads.
+// read-only for the launch (read-only path); x was written by the team's CTAs
+// earlier in the launch (before a barrier of the team), so it is read with
+// coherent loads.
 template <int VEC, bool S, class T>
 __device__ __forceinline__ T row_dot(const int *__restrict__ rp, const int *__restrict__ ci,
                                      const T *__restrict__ v, const T *x, int i, bool in, int l)
@@ -197,8 +198,8 @@ __device__ __forceinline__ int batch_check(const BatchCg &a, SysState &t, int sy
     return monitor_check(t, mon, r, a.hist_r + h, a.hist_it + h);
 }
 
-// CG + identity / Jacobi on rows [r0, r1): CgInit, then CgP, CgQ, CgUpd per
-// iteration (solver.cu), in one CTA
+// CG + identity / Jacobi on a system: CgInit, then CgP, CgQ, CgUpd per
+// iteration (solver.cu), by a team of which this CTA holds rows [r0, r1)
 template <int VEC, bool S, bool TM>
 __device__ void cg_system(const BatchCg &a, int sys, Shared &sh, int &turn)
 {
@@ -339,8 +340,9 @@ __device__ void cg_system(const BatchCg &a, int sys, Shared &sh, int &turn)
     }
 }
 
-// Mixed precision on rows [r0, r1): the outer step and inner FP32 CG of
-// phases.cuh (MxX, MxOuter, MxP, MxQ, MxUpd), in one CTA
+// Mixed precision on a system: the outer step and inner FP32 CG of phases.cuh
+// (MxX, MxOuter, MxP, MxQ, MxUpd), by a team of which this CTA holds rows
+// [r0, r1)
 template <int VEC, bool S, bool TM>
 __device__ void mixed_system(const BatchCg &a, int sys, Shared &sh, int &turn)
 {

@@ -914,10 +914,14 @@ void tile_drop32(TilePair *t)
 // Tiles of lines pay when rows form lines (kMinLine rows each on average), a
 // record holds every row (kLineK entries), the two triangles mirror each
 // other (so that one plan, walked up and down, serves both sweeps), the tiles
-// fit the SMs one each (none waits for a place), and the empty lanes stay
-// fewer than the rows.  Tiles: 128 lanes, 256 when 128 give more tiles than
-// SMs; among the shapes the one with the fewest tile boundaries on a path
-// across the grid.
+// fit the SMs one each (none waits for a place), and the plan has at most 2 n +
+// 65536 places (so a small system's lanes may be mostly empty: 1600 rows in
+// 27,648 places).  Tiles: 128 lanes, 256 when 128 give more tiles than SMs;
+// among the shapes the one with the fewest tile boundaries on a path across
+// the grid.  For cubes that is 128 lanes up to 128^3, 256 up to 192^3, and no
+// plan beyond.  ILU apply / setMatrix: 128^3 0.37 / 2.9 ms, 129^3 0.49 / 18.6
+// (256 lanes of three entries leave the pivots to the levels), 192^3 0.76 / 53,
+// 193^3 by levels 2.4 / 115 ms.
 static int tile_plan(mtjg_ctx *ctx, const TriOp &op, const TriOp &up, TilePlan **out)
 {
     *out = nullptr;

@@ -32,14 +32,18 @@
 
 // systems of at most this many product tiles take the one-launch CG (when
 // their tiles also fit the shared memory of the co-resident CTAs).  Measured
-// on GB300 (CG + Jacobi): 1.4-1.5x the graph path's speed up to ~100 tiles,
-// 1.2x at ~300, even at ~600 and behind it beyond.
+// on GB300 (CG + Jacobi, against the graph path): 2.0-2.6 times its speed up
+// to 150 tiles, 1.5 at 300 (one tile a CTA), 1.3-1.4 from 305 to 512 (two a
+// CTA: 2D 340^2 24.5 -> 17.8 ms, 3D 43^3 4.02 -> 2.84 ms).  A thread collects
+// the partials of two tiles for 512; with a limit of 608 (as many as two a CTA
+// hold) it collects three, and while systems of 513 to 608 tiles were 1.25
+// times as fast as the graph, those below lost up to a fifth (2D 340^2 20.2 ms,
+// 3D 36^3 2.02 -> 2.41 ms).
 #ifndef MTJG_PERSIST_MAX_TILES
 #define MTJG_PERSIST_MAX_TILES 512
 #endif
 // resident CTAs per SM the one-launch CG is compiled for (its register cap):
-// 2 (107 registers, no spills) measured a little faster than 3 or 4 at every
-// size
+// 2, which 90 to 96 registers and no spills need
 #ifndef MTJG_PERSIST_MINB
 #define MTJG_PERSIST_MINB 2
 #endif
