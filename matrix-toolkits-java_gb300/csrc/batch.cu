@@ -56,6 +56,7 @@ namespace cg = cooperative_groups;
 
 struct Shared {
     Acc warp_acc[kBatchBlock / 32];
+    double half[3][kBatchBlock / 2];  // per slot, each warp's sums after the first level
     Acc part[2];  // this CTA's partial, in two places by turns
     Acc out;
     SysState st;  // the system's state: every CTA of a team keeps the same
@@ -72,14 +73,23 @@ __device__ __forceinline__ void team_sync()
 }
 
 // Fixed-order reduction over the team: a fixed butterfly inside each warp,
-// then warps in order by thread 0, then the team's CTAs in rank order; the
-// result is broadcast through sh.out.
+// then warps in order, then the team's CTAs in rank order; the result is
+// broadcast through sh.out.
+//
+// Plain sums (every slot but the maximum and the robust norm): each warp does
+// the first level of its butterfly, and the other four levels of all eight
+// warps are one warp's per slot, whose lanes hold two warps' halves, then four
+// warps' quarters, then all eighths -- 8 + 5 + 7 FP64 additions a slot where a
+// butterfly in every warp takes 40 + 7, with the same pairs and the same order.
+// A team's CTA reduces as often as a whole system's for a share of its rows, so
+// on a full GPU the reductions were what teams cost.  With a butterfly a warp /
+// so, in ms: 1200 Laplacians of 6000 rows 23.8 / 22.0 (20.8 by one CTA a system),
+// 600 of 8300 rows 17.2 / 16.0, 300 2D Poisson grids 129^2 97.9 / 91.3 (mixed 77.1 /
+// 70.4), 600 grids 40^2, one CTA each, 7.35 / 6.10.
 template <int SLOTS, bool TM>
-__device__ __forceinline__ void team_reduce(Acc &a, int type, Shared &sh, int &turn)
+__device__ __forceinline__ void team_reduce_norm(Acc &a, int type, Shared &sh, int &turn)
 {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    if constexpr ((SLOTS & kSlotD2) != 0) a.v[2] += (double)a.f[0];
-    if constexpr ((SLOTS & kSlotD3) != 0) a.v[3] += (double)a.f[1];
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) acc_shfl_down<SLOTS>(a, off, type);
     if (lane == 0) sh.warp_acc[w] = a;
@@ -98,6 +108,62 @@ __device__ __forceinline__ void team_reduce(Acc &a, int type, Shared &sh, int &t
             for (int r = 1; r < (int)team.num_blocks(); ++r)
                 acc_merge_m<SLOTS>(s, *team.map_shared_rank(&sh.part[turn], r), type);
             sh.out = s;
+        }
+        turn ^= 1;
+    }
+    __syncthreads();
+}
+
+template <int SLOTS, bool TM>
+__device__ __forceinline__ void team_reduce(Acc &a, int type, Shared &sh, int &turn)
+{
+    if constexpr ((SLOTS & kSlotD2) != 0) a.v[2] += (double)a.f[0];
+    if constexpr ((SLOTS & kSlotD3) != 0) a.v[3] += (double)a.f[1];
+    if constexpr ((SLOTS & kSlotNorm) != 0) {
+        if (type != MTJG_NORM_ONE && type != MTJG_NORM_TWO) {
+            team_reduce_norm<SLOTS, TM>(a, type, sh, turn);
+            return;
+        }
+    }
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {  // slots 0, 2, 3
+        if (!(SLOTS & (i == 0 ? kSlotNorm : 2 << i))) continue;
+        const double v = a.v[i == 0 ? 0 : i + 1];
+        const double s = v + __shfl_down_sync(0xffffffffu, v, 16);
+        if (lane < 16) sh.half[i][w * 16 + lane] = s;
+    }
+    __syncthreads();
+    const int slot = w == 0 ? 0 : w + 1;
+    const bool mine = w < 3 && (SLOTS & (w == 0 ? kSlotNorm : 2 << w)) != 0;
+    if (mine) {
+        const double *h = &sh.half[w][lane & 15];
+        const int up = (lane >> 4) * 4;
+        double r[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) r[k] = h[(k + up) * 16];
+        const bool b8 = lane & 8, b4 = lane & 4;
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
+            r[k] = (b8 ? r[k + 2] : r[k]) + __shfl_xor_sync(0xffffffffu, b8 ? r[k] : r[k + 2], 8);
+        double v = (b4 ? r[1] : r[0]) + __shfl_xor_sync(0xffffffffu, b4 ? r[0] : r[1], 4);
+        v += __shfl_xor_sync(0xffffffffu, v, 2);
+        v += __shfl_xor_sync(0xffffffffu, v, 1);
+        double s = v;  // lane 0: warp 0's; warp k's in lane 16 (k / 4) + 8 (k / 2 % 2) + 4 (k % 2)
+#pragma unroll
+        for (int k = 1; k < kBatchBlock / 32; ++k)
+            s += __shfl_sync(0xffffffffu, v, (k & 4) * 4 + (k & 2) * 4 + (k & 1) * 4);
+        if (lane == 0) (TM ? sh.part[turn] : sh.out).v[slot] = s;
+    }
+    if constexpr (TM) {
+        team_sync<TM>();
+        if (mine) {
+            cg::cluster_group team = cg::this_cluster();
+            const int C = (int)team.num_blocks();
+            const double v = lane < C ? *team.map_shared_rank(&sh.part[turn].v[slot], lane) : 0.0;
+            double s = v;
+            for (int r = 1; r < C; ++r) s += __shfl_sync(0xffffffffu, v, r);
+            if (lane == 0) sh.out.v[slot] = s;
         }
         turn ^= 1;
     }

@@ -63,11 +63,12 @@ inline int64_t batch_makespan(const int *sys_rows, const int *order, int count, 
 // systems are left for it.  Three a SM are best where there are many rounds;
 // two where they need (almost) as many rounds as three: 300 systems of 6000
 // rows of 19 entries are two rounds by 228 teams of two and two by 152.
-// Measured, FP64, one CTA a system / three a SM / two, in ms: 300 such systems
-// 5.51 / 7.86 / 5.66; 300 of 4200 rows 3.92 / 5.26 / 4.20; 250 of 7000 rows
-// 6.32 / 8.47 / 6.49; 250 2D Poisson grids 90^2 31.8 / 36.8 / 30.3; 60 grids
-// 129^2 69.9 / 27.6 / 24.4.  Where two a SM need more rounds: 1200 systems of
-// 4200 rows 14.5 / 15.8 / 16.1, 300 of 17000 rows 16.3 / 17.7 / 20.0.
+// Measured, FP64, one CTA a system / three a SM / two, in ms (a butterfly per
+// warp in the reductions): 300 such systems 5.51 / 7.86 / 5.66; 300 of 4200 rows
+// 3.92 / 5.26 / 4.20; 250 of 7000 rows 6.32 / 8.47 / 6.49; 250 2D Poisson grids
+// 90^2 31.8 / 36.8 / 30.3; 60 grids 129^2 69.9 / 27.6 / 24.4.  Where two a SM need
+// more rounds: 1200 systems of 4200 rows 14.5 / 15.8 / 16.1, 300 of 17000 rows
+// 16.3 / 17.7 / 20.0.
 inline int batch_per_sm(const int *sys_rows, const int *order, int count, int team, int num_sms)
 {
     const int64_t three = (int64_t)kBatchPerSm * num_sms / team, two = (int64_t)2 * num_sms / team;
