@@ -55,8 +55,10 @@ namespace {
 namespace cg = cooperative_groups;
 
 struct Shared {
-    Acc warp_acc[kBatchBlock / 32];
-    double half[3][kBatchBlock / 2];  // per slot, each warp's sums after the first level
+    union {
+        Acc warp_acc[kBatchBlock / 32];
+        double quarter[2][kBatchBlock / 4];  // per slot, each warp's sums after two levels
+    };
     Acc part[2];  // this CTA's partial, in two places by turns
     Acc out;
     SysState st;  // the system's state: every CTA of a team keeps the same
@@ -76,18 +78,22 @@ __device__ __forceinline__ void team_sync()
 // then warps in order, then the team's CTAs in rank order; the result is
 // broadcast through sh.out.
 //
-// Plain sums (every slot but the maximum and the robust norm): each warp does
-// the first level of its butterfly, and the other four levels of all eight
-// warps are one warp's per slot, whose lanes hold two warps' halves, then four
-// warps' quarters, then all eighths -- 8 + 5 + 7 FP64 additions a slot where a
+// One or two plain sums (not the maximum or the robust norm, nor the three of
+// a refinement step): each warp does two levels of its butterfly, and one warp
+// per slot the other three of all eight warps, whose lanes hold four warps'
+// quarters, then all eighths -- 16 + 3 + 7 FP64 additions a slot where a
 // butterfly in every warp takes 40 + 7, with the same pairs and the same order.
 // A team's CTA reduces as often as a whole system's for a share of its rows, so
-// on a full GPU the reductions were what teams cost.  With a butterfly a warp /
-// so, in ms: 1200 Laplacians of 6000 rows 23.8 / 22.0 (20.8 by one CTA a system),
-// 600 of 8300 rows 17.2 / 16.0, 300 2D Poisson grids 129^2 97.9 / 91.3 (mixed 77.1 /
-// 70.4), 600 grids 40^2, one CTA each, 7.35 / 6.10.
+// on a full GPU the reductions were part of what teams cost.  With a butterfly a
+// warp / so, in ms: 300 2D Poisson grids 129^2 96.7 / 92.4 (mixed 75.5 / 69.8), 1200
+// grids 64^2 44.1 / 41.1 (30.2 / 27.2), 600 grids 40^2, one CTA each, 7.38 / 6.16,
+// 600 Laplacians of 8300 rows 17.1 / 16.7; 1024 grids of 32^2 to 256^2 376 / 368,
+// mixed 249 / 252.  One level a warp and four by one warp (20 additions) is
+// faster where the FP64 pipe is the bound (1200 Laplacians of 6000 rows 23.5 ->
+// 22.0) but takes 2.4 KB more shared memory a CTA, which the L1 then lacks (those
+// 1024 grids, mixed, 266).
 template <int SLOTS, bool TM>
-__device__ __forceinline__ void team_reduce_norm(Acc &a, int type, Shared &sh, int &turn)
+__device__ __forceinline__ void team_reduce_any(Acc &a, int type, Shared &sh, int &turn)
 {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
 #pragma unroll
@@ -119,40 +125,32 @@ __device__ __forceinline__ void team_reduce(Acc &a, int type, Shared &sh, int &t
 {
     if constexpr ((SLOTS & kSlotD2) != 0) a.v[2] += (double)a.f[0];
     if constexpr ((SLOTS & kSlotD3) != 0) a.v[3] += (double)a.f[1];
-    if constexpr ((SLOTS & kSlotNorm) != 0) {
-        if (type != MTJG_NORM_ONE && type != MTJG_NORM_TWO) {
-            team_reduce_norm<SLOTS, TM>(a, type, sh, turn);
-            return;
-        }
+    constexpr int kN = (SLOTS & kSlotNorm) ? 1 : 0, kD2 = (SLOTS & kSlotD2) ? 1 : 0, kD3 = (SLOTS & kSlotD3) ? 1 : 0;
+    if (kN + kD2 + kD3 > 2 || (kN && type != MTJG_NORM_ONE && type != MTJG_NORM_TWO)) {
+        team_reduce_any<SLOTS, TM>(a, type, sh, turn);
+        return;
     }
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    constexpr int kFirst = kN ? 0 : kD2 ? 2 : 3, kSecond = kN && kD2 ? 2 : 3;  // the slots, by warps 0 and 1
 #pragma unroll
-    for (int i = 0; i < 3; ++i) {  // slots 0, 2, 3
-        if (!(SLOTS & (i == 0 ? kSlotNorm : 2 << i))) continue;
-        const double v = a.v[i == 0 ? 0 : i + 1];
-        const double s = v + __shfl_down_sync(0xffffffffu, v, 16);
-        if (lane < 16) sh.half[i][w * 16 + lane] = s;
+    for (int i = 0; i < kN + kD2 + kD3 && i < 2; ++i) {
+        double v = a.v[i ? kSecond : kFirst];
+        v += __shfl_down_sync(0xffffffffu, v, 16);
+        v += __shfl_down_sync(0xffffffffu, v, 8);
+        if (lane < 8) sh.quarter[i][w * 8 + lane] = v;
     }
     __syncthreads();
-    const int slot = w == 0 ? 0 : w + 1;
-    const bool mine = w < 3 && (SLOTS & (w == 0 ? kSlotNorm : 2 << w)) != 0;
+    const int slot = w ? kSecond : kFirst;
+    const bool mine = w < kN + kD2 + kD3;
     if (mine) {
-        const double *h = &sh.half[w][lane & 15];
-        const int up = (lane >> 4) * 4;
-        double r[4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) r[k] = h[(k + up) * 16];
-        const bool b8 = lane & 8, b4 = lane & 4;
-#pragma unroll
-        for (int k = 0; k < 2; ++k)
-            r[k] = (b8 ? r[k + 2] : r[k]) + __shfl_xor_sync(0xffffffffu, b8 ? r[k] : r[k + 2], 8);
-        double v = (b4 ? r[1] : r[0]) + __shfl_xor_sync(0xffffffffu, b4 ? r[0] : r[1], 4);
+        const double lo = sh.quarter[w & 1][lane], hi = sh.quarter[w & 1][lane + 32];  // warps 0 to 3, 4 to 7
+        const bool b4 = lane & 4;
+        double v = (b4 ? hi : lo) + __shfl_xor_sync(0xffffffffu, b4 ? lo : hi, 4);
         v += __shfl_xor_sync(0xffffffffu, v, 2);
         v += __shfl_xor_sync(0xffffffffu, v, 1);
-        double s = v;  // lane 0: warp 0's; warp k's in lane 16 (k / 4) + 8 (k / 2 % 2) + 4 (k % 2)
+        double s = v;  // lane 0: warp 0's; warp k's in lane 8 (k % 4) + 4 (k / 4)
 #pragma unroll
-        for (int k = 1; k < kBatchBlock / 32; ++k)
-            s += __shfl_sync(0xffffffffu, v, (k & 4) * 4 + (k & 2) * 4 + (k & 1) * 4);
+        for (int k = 1; k < kBatchBlock / 32; ++k) s += __shfl_sync(0xffffffffu, v, (k & 3) * 8 + (k & 4));
         if (lane == 0) (TM ? sh.part[turn] : sh.out).v[slot] = s;
     }
     if constexpr (TM) {
