@@ -1114,7 +1114,7 @@ int tile_pair(mtjg_ctx *ctx, const TriOp &lo, const TriOp &up, TilePlan *plan, T
 // and not one per entry), then one pass over the entries.  96^3 convection-diffusion:
 // 4.2 ms by one launch per level (after 2.4 ms to find the levels), 0.86 ms
 // with a division per entry, 0.41 ms as here; setMatrix and one apply 17.6 ->
-// 3.05 ms, of which about 1 ms allocates and frees.
+// 2.4 ms.
 //
 // *other = 1 when some step finds another column (MTJ's scan, its read past
 // the row's end included).
